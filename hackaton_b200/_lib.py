@@ -22,6 +22,7 @@ EXPORTS = (
     "nf4b200_set_sm_limit", "nf4b200_gate_up_swiglu_fwd", "nf4b200_gate_up_swiglu_workspace_bytes",
     "nf4b200_swiglu_fwd", "nf4b200_swiglu_bwd", "nf4b200_linear_bwd_dx_swiglu",
     "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", "nf4b200_rmsnorm_fwd", "nf4b200_rmsnorm_bwd",
+    "nf4b200_add_rmsnorm_bwd",
     "nf4b200_qkv_rotate", "nf4b200_ce_stats", "nf4b200_ce_grad", "nf4b200_selftest_wait", "nf4b200_fp16_linear",
 )
 
@@ -116,6 +117,8 @@ def lib() -> ctypes.CDLL:
     handle.nf4b200_linear_bwd_dx_swiglu_workspace_bytes.restype = c_int64
     handle.nf4b200_rmsnorm_fwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                            c_void_p, c_int64, c_int64, c_float, c_void_p]
+    handle.nf4b200_add_rmsnorm_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                               c_void_p, c_void_p, c_int64, c_int64, c_void_p]
     handle.nf4b200_rmsnorm_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                            c_void_p, c_int64, c_int64, c_void_p]
     handle.nf4b200_qkv_rotate.argtypes = [c_void_p] * 8 + [c_int64, c_int64, c_void_p, c_void_p, c_int64,

@@ -692,6 +692,12 @@ int nf4b200_rmsnorm_fwd(const void* x, const void* delta, const void* weight, vo
 int nf4b200_rmsnorm_bwd(const void* x, const void* weight, const void* rstd, const void* dy,
                         int dy_dtype, const void* d_total, void* dx, int64_t rows, int64_t hidden,
                         void* stream) {
+    return nf4b200_add_rmsnorm_bwd(x, weight, rstd, dy, dy_dtype, d_total, dx, nullptr, rows, hidden, stream);
+}
+
+int nf4b200_add_rmsnorm_bwd(const void* x, const void* weight, const void* rstd, const void* dy,
+                            int dy_dtype, const void* d_total, void* dx, void* d_delta, int64_t rows,
+                            int64_t hidden, void* stream) {
     DeviceInfo* d = nullptr;
     int rc = require_sm100(&d);
     if (rc != NF4B200_OK) return rc;
@@ -704,7 +710,7 @@ int nf4b200_rmsnorm_bwd(const void* x, const void* weight, const void* rstd, con
     nf4::RmsNormArgs a = {};
     a.x = static_cast<const float*>(x); a.w = static_cast<const float*>(weight);
     a.rstd = const_cast<float*>(static_cast<const float*>(rstd));
-    a.dy = dy; a.dx = static_cast<float*>(dx); a.d_total = static_cast<const float*>(d_total);
+    a.dy = dy; a.dx = static_cast<float*>(dx); a.dx16 = d_delta; a.d_total = static_cast<const float*>(d_total);
     a.rows = rows; a.hidden = (int)hidden; a.mode = d_total ? 3 : 1;
     a.y_half = dy_dtype == NF4B200_F16 ? 1 : 0; a.eps = 0.f;
     cudaError_t e = nf4::launch_rmsnorm(a, static_cast<cudaStream_t>(stream));

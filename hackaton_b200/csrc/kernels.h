@@ -153,6 +153,7 @@ struct RmsNormArgs {
     float* rstd;           // [rows]: written by 0 / 2, read by 1 / 3
     const void* dy;        // modes 1, 3: gradient of y, same type as y
     float* dx;             // modes 1, 3
+    void* dx16;            // modes 1, 3: fp16 copy of dx, or null
     const void* delta;     // mode 2: fp16 [rows, hidden], added to x
     float* total;          // mode 2: x + delta
     const float* d_total;  // mode 3: gradient of the sum, added to dx

@@ -4,13 +4,23 @@
 //   1  backward           dx = rstd * (g - xhat * mean(g * xhat)),  g = dy * w, xhat = x * rstd
 //   2  add + forward      s = x + delta (delta fp16), s stored, then mode 0 on s
 //   3  backward + the gradient that reaches the sum directly: dx += d_total
-// x, w, s, dx, d_total fp32; y (and dy) fp32 or fp16 (the projections that follow read fp16).
-// One warp owns one row: the row is read once into registers with 16-byte loads that are all in
-// flight together (hidden = 128 * NV floats; NV = 12 and 28 are the Qwen2.5 1.5B / 7B widths),
-// two warp reductions by shuffles, outputs written once. HBM bound: 6 to 14 bytes per element.
-// Any other width takes the generic kernel, which walks the row twice (the second time out of
-// L1 / L2). Inputs are read through the read-only path (ld.global.nc), which lets the compiler
-// issue a row's loads ahead of its stores: outputs must not overlap inputs.
+// x, w, s, dx, d_total fp32; y (and dy) fp32 or fp16 (the projections that follow read fp16). Modes
+// 1 and 3 also write dx in fp16 where asked: the gradient of mode 2's delta, without a second pass
+// over dx (16,384 x 1536: 54 + 22 us as a kernel and a cast, 66 as one kernel).
+// HBM bound: 6 to 16 bytes per element. A row is read once into registers with 16-byte loads that
+// are all in flight together, and every output is written once. Who owns a row depends on what has
+// to be in flight (us measured, one CTA per row against one warp per row):
+//   forward, many rows of the 1.5B / 7B widths (1536, 3584): one warp; 16,384 x 3584 with the add
+//     105.6 against 113.7
+//   backward: one CTA with one float4 of each array per thread (mode 3, 16,384 x 1536 with the fp16
+//     copy: 65.8 against 68.8, where a warp's 12 to 28 float4 of two arrays spill) or two (mode 1: 43.7
+//     against 49.8)
+//   up to 512 rows, where latency counts: one CTA with one float4 per thread (64 x 3584 with the add
+//     2.7 against 5.8, 1 x 1536 1.7 against 1.9)
+//   other widths: one CTA. Before, these took the generic kernel (scalar accesses, the row walked
+//     twice), which is left for rows that are not whole float4 or longer than 16,384.
+// Inputs are read through the read-only path (ld.global.nc), which lets the compiler issue a row's
+// loads ahead of its stores: outputs must not overlap inputs.
 #include <cuda_fp16.h>
 
 #include "kernels.h"
@@ -48,7 +58,13 @@ __device__ __forceinline__ void store4_any(void* base, long long idx4, int half,
     }
 }
 
-template <int NV>
+__device__ __forceinline__ void store_dx(const RmsNormArgs& a, long long idx4, float4 dx) {
+    reinterpret_cast<float4*>(a.dx)[idx4] = dx;
+    if (a.dx16 != nullptr) store4_any(a.dx16, idx4, 1, dx);
+}
+
+// Forward over many rows: one warp per row.
+template <int NV, bool ADD>
 __global__ void __launch_bounds__(RN_WARPS * 32, NV <= 16 ? 2 : 1)
 rmsnorm_rows_kernel(const RmsNormArgs a) {
     grid_dep_wait();
@@ -60,7 +76,7 @@ rmsnorm_rows_kernel(const RmsNormArgs a) {
     float4 x[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) x[i] = __ldg(reinterpret_cast<const float4*>(a.x) + base4 + i * 32 + lane);
-    if (a.mode == 2) {
+    if (ADD) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const float4 d = load4_any(a.delta, base4 + i * 32 + lane, 1);
@@ -68,76 +84,103 @@ rmsnorm_rows_kernel(const RmsNormArgs a) {
             reinterpret_cast<float4*>(a.total)[base4 + i * 32 + lane] = x[i];
         }
     }
-    const float inv_h = 1.f / (float)(NV * 128);
-    if ((a.mode & 1) == 0) {
-        float ss = 0.f;
+    float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < NV; ++i)
-            ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
-        ss = warp_sum(ss);
-        const float rstd = 1.f / sqrtf(ss * inv_h + a.eps);
+    for (int i = 0; i < NV; ++i)
+        ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+    const float rstd = 1.f / sqrtf(warp_sum(ss) * (1.f / (float)(NV * 128)) + a.eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const float4 w = __ldg(reinterpret_cast<const float4*>(a.w) + i * 32 + lane);
+        store4_any(a.y, base4 + i * 32 + lane, a.y_half,
+                   make_float4(w.x * (x[i].x * rstd), w.y * (x[i].y * rstd),
+                               w.z * (x[i].z * rstd), w.w * (x[i].w * rstd)));
+    }
+    if (lane == 0) a.rstd[row] = rstd;
+}
+
+// Sum over the CTA, the same value in every thread.
+__device__ __forceinline__ float block_sum(float v) {
+    __shared__ float part[32];
+    v = warp_sum(v);
+    const int warps = blockDim.x >> 5;
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    const int l = threadIdx.x & 31;
+    return warp_sum(l < warps ? part[l] : 0.f);
+}
+
+// One CTA per row of hidden = 4 * h4 floats, NV float4 per thread; everything the row needs is
+// requested before the first value is used.
+template <int NV, int MODE>
+__global__ void __launch_bounds__(1024)
+rmsnorm_block_kernel(const RmsNormArgs a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    const int h4 = a.hidden >> 2;
+    const long long row = blockIdx.x, base4 = row * h4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x[NV], w[NV], d[NV], t[NV];   // d: mode 2 the delta, modes 1 and 3 dy; t: d_total
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        x[i] = w[i] = d[i] = t[i] = zero;
+        if (c < h4) {
+            x[i] = __ldg(reinterpret_cast<const float4*>(a.x) + base4 + c);
+            if (MODE == 1 || MODE == 3) d[i] = load4_any(a.dy, base4 + c, a.y_half);
+            if (MODE == 2) d[i] = load4_any(a.delta, base4 + c, 1);
+            if (MODE == 3) t[i] = __ldg(reinterpret_cast<const float4*>(a.d_total) + base4 + c);
+            w[i] = __ldg(reinterpret_cast<const float4*>(a.w) + c);
+        }
+    }
+    const float inv_h = 1.f / (float)a.hidden;
+    float sum = 0.f;
+    if (MODE == 0 || MODE == 2) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(a.w) + i * 32 + lane);
-            store4_any(a.y, base4 + i * 32 + lane, a.y_half,
-                       make_float4(w.x * (x[i].x * rstd), w.y * (x[i].y * rstd),
-                                   w.z * (x[i].z * rstd), w.w * (x[i].w * rstd)));
+            if (MODE == 2) { x[i].x += d[i].x; x[i].y += d[i].y; x[i].z += d[i].z; x[i].w += d[i].w; }
+            sum += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
         }
-        if (lane == 0) a.rstd[row] = rstd;
-    } else {
-        const float rstd = a.rstd[row];
-        float dot = 0.f;
-        if (a.y_half && NV <= 16) {
-            // fp16 dy of a narrow row stays in registers (2 per 4 elements) next to xhat
-            uint2 dyr[NV];
-#pragma unroll
-            for (int i = 0; i < NV; ++i) dyr[i] = __ldg(reinterpret_cast<const uint2*>(a.dy) + base4 + i * 32 + lane);
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const float4 w = __ldg(reinterpret_cast<const float4*>(a.w) + i * 32 + lane);
-                const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&dyr[i].x));
-                const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&dyr[i].y));
-                x[i].x *= rstd; x[i].y *= rstd; x[i].z *= rstd; x[i].w *= rstd;  // xhat
-                dot += lo.x * w.x * x[i].x + lo.y * w.y * x[i].y + hi.x * w.z * x[i].z + hi.y * w.w * x[i].w;
-            }
-            const float mean_gx = warp_sum(dot) * inv_h;
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const float4 w = __ldg(reinterpret_cast<const float4*>(a.w) + i * 32 + lane);
-                const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&dyr[i].x));
-                const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&dyr[i].y));
-                float4 dx = make_float4(rstd * (lo.x * w.x - x[i].x * mean_gx), rstd * (lo.y * w.y - x[i].y * mean_gx),
-                                        rstd * (hi.x * w.z - x[i].z * mean_gx), rstd * (hi.y * w.w - x[i].w * mean_gx));
-                if (a.mode == 3) {
-                    const float4 t = __ldg(reinterpret_cast<const float4*>(a.d_total) + base4 + i * 32 + lane);
-                    dx.x += t.x; dx.y += t.y; dx.z += t.z; dx.w += t.w;
-                }
-                reinterpret_cast<float4*>(a.dx)[base4 + i * 32 + lane] = dx;
-            }
-            return;
-        }
-        // otherwise the row of dy is read twice (the second time out of L1 / L2): keeping it next
-        // to xhat would need up to 2 * NV float4 registers per thread
+        const float rstd = 1.f / sqrtf(block_sum(sum) * inv_h + a.eps);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(a.w) + i * 32 + lane);
-            const float4 dy = load4_any(a.dy, base4 + i * 32 + lane, a.y_half);
-            x[i].x *= rstd; x[i].y *= rstd; x[i].z *= rstd; x[i].w *= rstd;  // xhat
-            dot += dy.x * w.x * x[i].x + dy.y * w.y * x[i].y + dy.z * w.z * x[i].z + dy.w * w.w * x[i].w;
+            const int c = threadIdx.x + i * blockDim.x;
+            if (c >= h4) continue;
+            if (MODE == 2) reinterpret_cast<float4*>(a.total)[base4 + c] = x[i];
+            store4_any(a.y, base4 + c, a.y_half,
+                       make_float4(w[i].x * (x[i].x * rstd), w[i].y * (x[i].y * rstd),
+                                   w[i].z * (x[i].z * rstd), w[i].w * (x[i].w * rstd)));
         }
-        const float mean_gx = warp_sum(dot) * inv_h;
+        if (threadIdx.x == 0) a.rstd[row] = rstd;
+        return;
+    }
+    const float rstd = a.rstd[row];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(a.w) + i * 32 + lane);
-            const float4 dy = load4_any(a.dy, base4 + i * 32 + lane, a.y_half);
-            float4 dx = make_float4(rstd * (dy.x * w.x - x[i].x * mean_gx), rstd * (dy.y * w.y - x[i].y * mean_gx),
-                                    rstd * (dy.z * w.z - x[i].z * mean_gx), rstd * (dy.w * w.w - x[i].w * mean_gx));
-            if (a.mode == 3) {
-                const float4 t = __ldg(reinterpret_cast<const float4*>(a.d_total) + base4 + i * 32 + lane);
-                dx.x += t.x; dx.y += t.y; dx.z += t.z; dx.w += t.w;
-            }
-            reinterpret_cast<float4*>(a.dx)[base4 + i * 32 + lane] = dx;
-        }
+    for (int i = 0; i < NV; ++i) {
+        x[i].x *= rstd; x[i].y *= rstd; x[i].z *= rstd; x[i].w *= rstd;              // xhat
+        d[i].x *= w[i].x; d[i].y *= w[i].y; d[i].z *= w[i].z; d[i].w *= w[i].w;      // g
+        sum += d[i].x * x[i].x + d[i].y * x[i].y + d[i].z * x[i].z + d[i].w * x[i].w;
+    }
+    const float mean_gx = block_sum(sum) * inv_h;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < h4)
+            store_dx(a, base4 + c, make_float4(rstd * (d[i].x - x[i].x * mean_gx) + t[i].x,
+                                               rstd * (d[i].y - x[i].y * mean_gx) + t[i].y,
+                                               rstd * (d[i].z - x[i].z * mean_gx) + t[i].z,
+                                               rstd * (d[i].w - x[i].w * mean_gx) + t[i].w));
+    }
+}
+
+template <int NV>
+static cudaError_t launch_block(const RmsNormArgs& a, cudaStream_t stream) {
+    const dim3 grid((unsigned)a.rows), block((unsigned)((a.hidden / 4 + 32 * NV - 1) / (32 * NV) * 32));
+    switch (a.mode) {
+        case 0: return launch_pdl(rmsnorm_block_kernel<NV, 0>, grid, block, 0, stream, a);
+        case 1: return launch_pdl(rmsnorm_block_kernel<NV, 1>, grid, block, 0, stream, a);
+        case 2: return launch_pdl(rmsnorm_block_kernel<NV, 2>, grid, block, 0, stream, a);
+        default: return launch_pdl(rmsnorm_block_kernel<NV, 3>, grid, block, 0, stream, a);
     }
 }
 
@@ -183,6 +226,7 @@ rmsnorm_generic_kernel(const RmsNormArgs a) {
             float dx = rstd * (dy * a.w[c] - xs[c] * rstd * mean_gx);
             if (a.mode == 3) dx += a.d_total[base + c];
             a.dx[base + c] = dx;
+            if (a.dx16 != nullptr) static_cast<__half*>(a.dx16)[base + c] = __float2half_rn(dx);
         }
     }
 }
@@ -193,11 +237,23 @@ cudaError_t launch_rmsnorm(const RmsNormArgs& a, cudaStream_t stream) {
     const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) |
                            reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.dy) |
                            reinterpret_cast<uintptr_t>(a.dx) | reinterpret_cast<uintptr_t>(a.delta) |
-                           reinterpret_cast<uintptr_t>(a.total) | reinterpret_cast<uintptr_t>(a.d_total);
+                           reinterpret_cast<uintptr_t>(a.total) | reinterpret_cast<uintptr_t>(a.d_total) |
+                           reinterpret_cast<uintptr_t>(a.dx16);
     const bool vec = (bits & 15) == 0;
-    if (vec && a.hidden == 12 * 128) return launch_pdl(rmsnorm_rows_kernel<12>, grid, block, 0, stream, a);
-    if (vec && a.hidden == 28 * 128) return launch_pdl(rmsnorm_rows_kernel<28>, grid, block, 0, stream, a);
-    return launch_pdl(rmsnorm_generic_kernel, grid, block, 0, stream, a);
+    const int h4 = a.hidden / 4;
+    if (!vec || a.hidden % 4 != 0 || a.rows > 0x7FFFFFFF || h4 > 4096)
+        return launch_pdl(rmsnorm_generic_kernel, grid, block, 0, stream, a);
+    const bool few = a.rows <= 512, backward = (a.mode & 1) != 0;
+    if (!few && !backward && a.hidden == 12 * 128)
+        return a.mode == 2 ? launch_pdl(rmsnorm_rows_kernel<12, true>, grid, block, 0, stream, a)
+                           : launch_pdl(rmsnorm_rows_kernel<12, false>, grid, block, 0, stream, a);
+    if (!few && !backward && a.hidden == 28 * 128)
+        return a.mode == 2 ? launch_pdl(rmsnorm_rows_kernel<28, true>, grid, block, 0, stream, a)
+                           : launch_pdl(rmsnorm_rows_kernel<28, false>, grid, block, 0, stream, a);
+    // float4 per thread: one where latency counts or four arrays are in flight, otherwise two
+    if (h4 <= 1024 && (few || a.mode == 3 || h4 <= 128)) return launch_block<1>(a, stream);
+    if (h4 <= 2048 && (few || backward || h4 <= 256)) return launch_block<2>(a, stream);
+    return launch_block<4>(a, stream);
 }
 
 }  // namespace nf4

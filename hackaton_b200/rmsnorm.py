@@ -35,16 +35,17 @@ def launch_forward(x2, delta2, weight, eps, to_half):
     return out, rstd, total
 
 
-def launch_backward(x2, weight, rstd, dy2, d_total=None):
+def launch_backward(x2, weight, rstd, dy2, d_total=None, dx16=None):
     """Gradient with respect to the normalised rows' input; `d_total` (fp32, optional) is added in
-    the same pass (the gradient that reached the sum directly)."""
+    the same pass (the gradient that reached the sum directly), `dx16` (optional) a contiguous fp16
+    tensor that receives the result's rounding."""
     rows, hidden = x2.shape
     dx = torch.empty_like(x2)
     with torch.cuda.device(x2.device):
-        _lib.check(_lib.lib().nf4b200_rmsnorm_bwd(
+        _lib.check(_lib.lib().nf4b200_add_rmsnorm_bwd(
             x2.data_ptr(), weight.data_ptr(), rstd.data_ptr(), dy2.data_ptr(), _out_code(dy2.dtype),
-            None if d_total is None else d_total.data_ptr(), dx.data_ptr(), rows, hidden,
-            _stream_ptr(x2.device)))
+            None if d_total is None else d_total.data_ptr(), dx.data_ptr(),
+            None if dx16 is None else dx16.data_ptr(), rows, hidden, _stream_ptr(x2.device)))
     return dx
 
 
@@ -90,12 +91,15 @@ class _NormOp:
         else:
             (dy,), d_total = grads, None
         dy2 = dy.reshape(rows.shape).contiguous()
-        dx = launch_backward(rows, weight, rstd, dy2, d_total).reshape(kept.shape)
+        dx16 = None
+        if self.with_delta and kept.wants[2]:
+            dx16 = torch.empty_like(rows, dtype=torch.float16)
+        dx = launch_backward(rows, weight, rstd, dy2, d_total, dx16).reshape(kept.shape)
         dweight = None
         if kept.wants[1]:
             dweight = (dy2.float() * (rows * rstd[:, None])).sum(dim=0).to(weight.dtype)
         if self.with_delta:
-            return dx, dweight, dx.to(torch.float16)
+            return dx, dweight, None if dx16 is None else dx16.reshape(kept.shape)
         return dx, dweight
 
 

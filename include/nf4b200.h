@@ -281,6 +281,11 @@ int nf4b200_rmsnorm_fwd(const void* x, const void* delta, const void* weight, vo
 int nf4b200_rmsnorm_bwd(const void* x, const void* weight, const void* rstd, const void* dy,
                         int dy_dtype, const void* d_total, void* dx, int64_t rows, int64_t hidden,
                         void* stream);
+/* The same with dx also written in fp16 (rounded to nearest) to d_delta, the gradient of the forward
+ * pass's fp16 delta; d_delta may be NULL. */
+int nf4b200_add_rmsnorm_bwd(const void* x, const void* weight, const void* rstd, const void* dy,
+                            int dy_dtype, const void* d_total, void* dx, void* d_delta, int64_t rows,
+                            int64_t hidden, void* stream);
 
 /*
  * Rotary embedding + grouped-query expansion on the packed q / k / v projections: the step after

@@ -112,3 +112,37 @@ def test_empty_and_errors(cuda_lib):
         rms_norm(torch.zeros(2, 1536, device="cuda").half(), w, 1e-6)
     with pytest.raises(ValueError):
         rms_norm(torch.zeros(2, 1024, device="cuda"), w, 1e-6)
+
+
+@pytest.mark.parametrize("rows", [1, 512, 513])                     # one CTA per row up to 512 rows
+@pytest.mark.parametrize("hidden", [4, 132, 640, 1536, 3192, 3584, 4100, 8196, 16388])
+def test_widths_and_row_counts(cuda_lib, rows, hidden):
+    """Every kernel the launcher picks (row per warp, row per CTA with 1, 2, 4, 8 loads per thread,
+    walked twice beyond 16,384), all four modes, against 64-bit arithmetic. fp32 bound: a sum of
+    `hidden` squares in any order is off by at most hidden * 2^-24 relative; in practice far less.
+    fp16 outputs: one rounding (2^-11)."""
+    from hackaton_b200.rmsnorm import launch_backward, launch_forward
+
+    g = torch.Generator(device="cuda").manual_seed(rows + hidden)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, d_total, delta = rand(rows, hidden), rand(rows, hidden), rand(rows, hidden).half()
+    weight, eps = rand(hidden) * 0.1 + 1, 1e-6
+    close = lambda a, b, t: torch.testing.assert_close(a.double(), b, rtol=t, atol=t)  # noqa: E731
+    for half in (True, False):
+        tol = 2.0 ** -10 if half else 1e-5
+        for with_delta in (True, False):
+            out, rstd, total = launch_forward(x, delta if with_delta else None, weight, eps, half)
+            s = x.double() + delta.double() if with_delta else x.double()
+            want_rstd = torch.rsqrt(s.square().mean(-1, keepdim=True) + eps)
+            close(rstd[:, None], want_rstd, 1e-5)
+            close(out, weight.double() * s * want_rstd, tol)
+            if with_delta:
+                close(total, s, 1e-6)
+        dy = rand(rows, hidden).to(out.dtype)
+        hat, gg = s * want_rstd, dy.double() * weight.double()
+        dx = want_rstd * (gg - hat * (gg * hat).mean(-1, keepdim=True))
+        close(launch_backward(x, weight, rstd, dy), dx, 2e-5)
+        dx16 = torch.empty_like(delta)
+        got = launch_backward(x, weight, rstd, dy, d_total, dx16)
+        close(got, dx + d_total.double(), 2e-5)
+        assert torch.equal(dx16, got.half())
