@@ -5,9 +5,12 @@
 //     the softmax (lse - E[x]) and the first index of the maximum. No fp32 copy of the logits.
 //   gradient:   grad = scale * (softmax - onehot(target)), 0 for rows with target < 0; may be
 //     written over the logits themselves (every element is read before it is replaced).
-// One CTA of 256 threads per row (a row of Qwen2.5's 151,936 logits is 297 KB), 16-byte loads.
+// Statistics: one CTA per row (a row of Qwen2.5's 151,936 logits is 297 KB), 16-byte loads, its
+// size chosen by the number of rows (launch_ce). Gradient: a CTA per 8192 logits of a row.
 // A thread rescales its running sums once per 8 logits (when their maximum beats the running
-// one), not once per logit, and works in the base-2 domain (one FMA + one ex2 per logit). HBM bound: 2 bytes per logit for the statistics, 4 for the gradient.
+// one), not once per logit, and works in the base-2 domain (one FMA + one ex2 per logit). HBM bound:
+// 2 bytes per logit for the statistics (where the arithmetic is close behind: 104 us without the
+// ex2, 95 at the copy bandwidth), 4 for the gradient.
 #include <cuda_fp16.h>
 
 #include "kernels.h"
@@ -15,7 +18,9 @@
 
 namespace nf4 {
 
-constexpr int CE_THREADS = 256;
+constexpr int CE_THREADS = 256;        // gradient
+constexpr int CE_GRAD_VECS = 4;         // 8-logit vectors per thread of the gradient
+constexpr int CE_STATS_VECS = 4;        // ... requested ahead by the statistics
 constexpr float CE_NEG = -1.0e30f;  // finite "minus infinity", as in the reference (kernels.py:36)
 
 // Running statistics of the logits seen so far, kept in the base-2 domain so that a logit costs
@@ -49,45 +54,53 @@ __device__ __forceinline__ CeState ce_merge(const CeState& a, const CeState& b) 
     return r;
 }
 
+// Eight logits as they lie in memory, and as floats.
 template <bool F32>
-__device__ __forceinline__ void ce_load8(const void* row, long long i, float (&x)[8]) {
-    if (F32) {
-        const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(row) + i);
-        const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(row) + i + 4);
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    } else {
-        const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const __half*>(row) + i);
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+struct CeRaw {
+    uint4 q[F32 ? 2 : 1];
+    __device__ __forceinline__ void load(const void* row, long long i) {
+        const uint4* p = reinterpret_cast<const uint4*>(static_cast<const char*>(row) + i * (F32 ? 4 : 2));
+        q[0] = p[0];
+        if (F32) q[F32 ? 1 : 0] = p[1];
+    }
+    __device__ __forceinline__ void unpack(float (&x)[8]) const {
+        if (F32) {
+            const uint32_t w[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[F32 ? 1 : 0].x, q[F32 ? 1 : 0].y,
+                                   q[F32 ? 1 : 0].z, q[F32 ? 1 : 0].w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-            x[2 * e] = f.x;
-            x[2 * e + 1] = f.y;
+            for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(w[e]);
+        } else {
+            const uint32_t w[4] = {q[0].x, q[0].y, q[0].z, q[0].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                x[2 * e] = f.x;
+                x[2 * e + 1] = f.y;
+            }
         }
     }
-}
+};
 
 template <bool F32>
 __device__ __forceinline__ float ce_load1(const void* row, long long i) {
     return F32 ? static_cast<const float*>(row)[i] : __half2float(static_cast<const __half*>(row)[i]);
 }
 
-template <bool F32>
-__global__ void __launch_bounds__(CE_THREADS)
+template <bool F32, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 ce_stats_kernel(const CeArgs a) {
     grid_dep_wait();
     grid_dep_launch();
-    __shared__ CeState part[CE_THREADS / 32];
+    __shared__ CeState part[THREADS / 32];
     const long long row = blockIdx.x;
     const void* base = F32 ? static_cast<const void*>(static_cast<const float*>(a.logits) + row * a.vocab)
                            : static_cast<const void*>(static_cast<const __half*>(a.logits) + row * a.vocab);
     CeState st = {CE_NEG, CE_NEG * CE_LOG2E, 0.f, 0.f, 0};
     const bool vec = a.vec != 0;
     const long long n8 = vec ? a.vocab / 8 : 0;
-#pragma unroll 4
-    for (long long v = threadIdx.x; v < n8; v += CE_THREADS) {
+    auto take = [&](const CeRaw<F32>& raw, long long v) {
         float x[8];
-        ce_load8<F32>(base, v * 8, x);
+        raw.unpack(x);
         float lm = x[0];
 #pragma unroll
         for (int e = 1; e < 8; ++e) lm = fmaxf(lm, x[e]);
@@ -111,8 +124,28 @@ ce_stats_kernel(const CeArgs a) {
             st.s += w;
             st.d = fmaf(w, t, st.d);
         }
+    };
+    // the next CE_STATS_VECS vectors are on their way while these are taken in
+    CeRaw<F32> next[CE_STATS_VECS];
+    long long v = threadIdx.x;
+    const auto fetch = [&](long long v0) {
+#pragma unroll
+        for (int u = 0; u < CE_STATS_VECS; ++u)
+            if (v0 + u * THREADS < n8) next[u].load(base, (v0 + u * THREADS) * 8);
+    };
+    fetch(v);
+    for (; v + (CE_STATS_VECS - 1) * THREADS < n8; v += CE_STATS_VECS * THREADS) {
+        CeRaw<F32> now[CE_STATS_VECS];
+#pragma unroll
+        for (int u = 0; u < CE_STATS_VECS; ++u) now[u] = next[u];
+        fetch(v + CE_STATS_VECS * THREADS);
+#pragma unroll
+        for (int u = 0; u < CE_STATS_VECS; ++u) take(now[u], v + u * THREADS);
     }
-    for (long long i = n8 * 8 + threadIdx.x; i < a.vocab; i += CE_THREADS) {
+#pragma unroll
+    for (int u = 0; u < CE_STATS_VECS; ++u)
+        if (v + u * THREADS < n8) take(next[u], v + u * THREADS);
+    for (long long i = n8 * 8 + threadIdx.x; i < a.vocab; i += THREADS) {
         const float x = ce_load1<F32>(base, i);
         if (x > st.m) {
             const float x2 = x * CE_LOG2E, t = st.m2 - x2;
@@ -142,7 +175,7 @@ ce_stats_kernel(const CeArgs a) {
     __syncthreads();
     if (threadIdx.x == 0) {
         CeState t = part[0];
-        for (int w = 1; w < CE_THREADS / 32; ++w) t = ce_merge(t, part[w]);
+        for (int w = 1; w < THREADS / 32; ++w) t = ce_merge(t, part[w]);
         // A target beyond the vocabulary (a tokenizer / padding mismatch) is treated like an
         // ignored row, its logit is never read, and the device status word records it.
         const long long target = a.targets[row];
@@ -158,61 +191,74 @@ ce_stats_kernel(const CeArgs a) {
     }
 }
 
+// A CTA handles CE_GRAD_VECS * 8 * 256 consecutive logits of a row (and the row's last CTA the
+// remainder that is no whole vector). Short CTAs in row order leave no partly filled last wave, and
+// the logits wait in registers as they lie in memory (34 registers), so that an SM holds enough of
+// them: 2048 x 151,936 fp16 184 us = 1.03 of the copy bandwidth; one 256-thread CTA per row, 1.7
+// waves, took 235.
 template <bool F32>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(const CeArgs a) {
     grid_dep_wait();
     grid_dep_launch();
-    const long long row = blockIdx.x;
+    const long long row = blockIdx.x / a.segments, segment = blockIdx.x % a.segments;
+    const void* base = F32 ? static_cast<const void*>(static_cast<const float*>(a.logits) + row * a.vocab)
+                           : static_cast<const void*>(static_cast<const __half*>(a.logits) + row * a.vocab);
+    void* out = F32 ? static_cast<void*>(static_cast<float*>(a.grad) + row * a.vocab)
+                    : static_cast<void*>(static_cast<__half*>(a.grad) + row * a.vocab);
+    const long long n8 = a.vec ? a.vocab / 8 : 0;
+    const long long v0 = segment * (CE_GRAD_VECS * CE_THREADS) + threadIdx.x;
+    // all loads go out before the first store (the output may be the input array, so the compiler
+    // has to keep loads behind earlier stores)
+    CeRaw<F32> raw[CE_GRAD_VECS];
+#pragma unroll
+    for (int u = 0; u < CE_GRAD_VECS; ++u)
+        if (v0 + u * CE_THREADS < n8) raw[u].load(base, (v0 + u * CE_THREADS) * 8);
     const long long target = a.targets[row];
     const float lse = a.lse[row];
     // ignored rows and rows whose target lies beyond the vocabulary get exact zeros (their lse
     // is 0: exp may overflow)
     const bool valid = target >= 0 && target < a.vocab;
     const float scale = *a.scale;
-    const void* base = F32 ? static_cast<const void*>(static_cast<const float*>(a.logits) + row * a.vocab)
-                           : static_cast<const void*>(static_cast<const __half*>(a.logits) + row * a.vocab);
-    void* out = F32 ? static_cast<void*>(static_cast<float*>(a.grad) + row * a.vocab)
-                    : static_cast<void*>(static_cast<__half*>(a.grad) + row * a.vocab);
-    const long long n8 = a.vec ? a.vocab / 8 : 0;
-    // four vectors per thread and step: their loads go out before the first store (the output may
-    // be the input array, so the compiler has to keep loads behind earlier stores)
-    for (long long v0 = threadIdx.x; v0 < n8; v0 += 4 * CE_THREADS) {
-        float x[4][8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (v0 + u * CE_THREADS < n8) ce_load8<F32>(base, (v0 + u * CE_THREADS) * 8, x[u]);
+    for (int u = 0; u < CE_GRAD_VECS; ++u) {
+        const long long v = v0 + u * CE_THREADS;
+        if (v >= n8) break;
+        float x[8], g[8];
+        raw[u].unpack(x);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const long long v = v0 + u * CE_THREADS;
-            if (v >= n8) break;
-            float g[8];
+        for (int e = 0; e < 8; ++e) {
+            const float hot = (v * 8 + e == target) ? 1.f : 0.f;
+            g[e] = valid ? (__expf(x[e] - lse) - hot) * scale : 0.f;
+        }
+        if (F32) {
+            float* o = static_cast<float*>(out) + v * 8;
+            *reinterpret_cast<float4*>(o) = make_float4(g[0], g[1], g[2], g[3]);
+            *reinterpret_cast<float4*>(o + 4) = make_float4(g[4], g[5], g[6], g[7]);
+        } else {
+            uint32_t w[4];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float hot = (v * 8 + e == target) ? 1.f : 0.f;
-                g[e] = valid ? (__expf(x[u][e] - lse) - hot) * scale : 0.f;
+            for (int e = 0; e < 4; ++e) {
+                const __half2 h = __floats2half2_rn(g[2 * e], g[2 * e + 1]);
+                w[e] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            if (F32) {
-                float* o = static_cast<float*>(out) + v * 8;
-                *reinterpret_cast<float4*>(o) = make_float4(g[0], g[1], g[2], g[3]);
-                *reinterpret_cast<float4*>(o + 4) = make_float4(g[4], g[5], g[6], g[7]);
-            } else {
-                uint32_t w[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const __half2 h = __floats2half2_rn(g[2 * e], g[2 * e + 1]);
-                    w[e] = *reinterpret_cast<const uint32_t*>(&h);
-                }
-                *reinterpret_cast<uint4*>(static_cast<__half*>(out) + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
+            *reinterpret_cast<uint4*>(static_cast<__half*>(out) + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
+    if (segment != a.segments - 1) return;
     for (long long i = n8 * 8 + threadIdx.x; i < a.vocab; i += CE_THREADS) {
-        const float x = ce_load1<F32>(base, i);
-        const float g = valid ? (__expf(x - lse) - (i == target ? 1.f : 0.f)) * scale : 0.f;
+        const float x1 = ce_load1<F32>(base, i);
+        const float g = valid ? (__expf(x1 - lse) - (i == target ? 1.f : 0.f)) * scale : 0.f;
         if (F32) static_cast<float*>(out)[i] = g;
         else     static_cast<__half*>(out)[i] = __float2half_rn(g);
     }
+}
+
+template <int THREADS>
+static cudaError_t launch_stats(const CeArgs& a, cudaStream_t stream) {
+    const dim3 grid((unsigned)a.rows), block(THREADS);
+    return a.f32 ? launch_pdl(ce_stats_kernel<true, THREADS>, grid, block, 0, stream, a)
+                 : launch_pdl(ce_stats_kernel<false, THREADS>, grid, block, 0, stream, a);
 }
 
 cudaError_t launch_ce(const CeArgs& a_in, cudaStream_t stream) {
@@ -222,12 +268,20 @@ cudaError_t launch_ce(const CeArgs& a_in, cudaStream_t stream) {
     // 16-byte accesses need every row to start on a 16-byte boundary
     a.vec = ((reinterpret_cast<uintptr_t>(a.logits) | reinterpret_cast<uintptr_t>(a.grad)) % 16 == 0 &&
              (a.vocab * elem) % 16 == 0) ? 1 : 0;
-    const dim3 grid((unsigned)a.rows), block(CE_THREADS);
-    if (a.grad != nullptr)
+    if (a.grad != nullptr) {
+        // rows without 16-byte accesses are walked by one CTA each
+        a.segments = a.vec ? (a.vocab / 8 + CE_GRAD_VECS * CE_THREADS - 1) / (CE_GRAD_VECS * CE_THREADS) : 1;
+        if (a.segments < 1) a.segments = 1;
+        const dim3 grid((unsigned)(a.rows * a.segments)), block(CE_THREADS);
         return a.f32 ? launch_pdl(ce_grad_kernel<true>, grid, block, 0, stream, a)
                      : launch_pdl(ce_grad_kernel<false>, grid, block, 0, stream, a);
-    return a.f32 ? launch_pdl(ce_stats_kernel<true>, grid, block, 0, stream, a)
-                 : launch_pdl(ce_stats_kernel<false>, grid, block, 0, stream, a);
+    }
+    // Threads per row: small CTAs for many rows leave the shortest last wave (2048 rows: 128 threads
+    // 116 us, 256: 121, 512: 127; before, with 256 threads and no loads ahead, 127), large ones give
+    // few rows enough loads in flight (256 rows: 512 threads 24 us, 1024: 28).
+    if (a.rows > 8 * 148) return launch_stats<128>(a, stream);
+    if (a.rows > 4 * 148) return launch_stats<256>(a, stream);
+    return launch_stats<512>(a, stream);
 }
 
 }  // namespace nf4

@@ -16,7 +16,12 @@ from ._autograd import call
 from .dense import fp16_linear
 from .nf4 import _stream_ptr
 
-CHUNK_ROWS = 256      # rows of logits alive at a time (solution/lm_loss.py:27)
+# Most rows of logits alive at a time. The reference holds 256 (solution/lm_loss.py:27) to fit 16 GB;
+# every chunk reads the whole head weight twice, so on a GPU with 180 GB more rows per chunk pay:
+# 2048 x 151,936 from 1536 takes 8 x 283 us in chunks of 256, 4 x 466 of 512, 2 x 864 of 1024 and
+# 1664 in one (622 MB of fp16 logits).
+CHUNK_ROWS = 2048
+CHUNK_TILE = 512      # token rows of the GEMM's largest tile
 GRAD_SCALE = 1024.0   # the chunk gradients are kept in fp16 at this scale (solution/lm_loss.py:28)
 
 
@@ -101,6 +106,16 @@ def _head_products(hidden_rows, weight):
             lambda d_logits, out: torch.mm(d_logits, weight, out=out))
 
 
+def _chunks(rows):
+    """Row slices of at most CHUNK_ROWS rows, of about equal size (no short last one, which would
+    read the whole weight for a few rows), whole tiles except for the last."""
+    if rows == 0:
+        return []
+    count = -(-rows // CHUNK_ROWS)
+    step = min(CHUNK_ROWS, -(-rows // (count * CHUNK_TILE)) * CHUNK_TILE)
+    return [slice(lo, min(lo + step, rows)) for lo in range(0, rows, step)]
+
+
 class _HeadAndLoss:
     """lm_head + loss without ever holding the (tokens, vocab) logits: walks the rows in chunks;
     per chunk the logits are made, reduced to their statistics, turned in place into
@@ -116,8 +131,7 @@ class _HeadAndLoss:
         d_hidden = torch.empty_like(hidden)
         unit = torch.full((1,), GRAD_SCALE, dtype=torch.float32, device=device)
         with torch.autocast("cuda", enabled=False):
-            for lo in range(0, rows, CHUNK_ROWS):
-                rs = slice(lo, min(lo + CHUNK_ROWS, rows))
+            for rs in _chunks(rows):
                 logits, back = _head_products(hidden[rs], weight)
                 ce_stats(logits, targets[rs], True,
                          out=(stats["lse"][rs], stats["loss"][rs], stats["entropy"][rs], argmax[rs]))

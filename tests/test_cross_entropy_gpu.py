@@ -96,3 +96,60 @@ def test_linear_cross_entropy_matches_unchunked(cuda_lib):
     torch.testing.assert_close(entropy.cpu(), o[2], rtol=1e-3, atol=1e-3)
     torch.testing.assert_close(hidden.grad.float(), ref_grad.float(), rtol=2e-2, atol=2e-6)
     cuda_lib.device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("rows", [3, 593, 1185])                       # 512, 256 and 128 threads per row
+@pytest.mark.parametrize("vocab", [1, 8, 1023, 8192, 8200, 16392])     # below, at and past a CTA's 8192 logits
+def test_thread_counts_and_segments(cuda_lib, rows, vocab, dtype):
+    """Every kernel the launcher picks, statistics and in-place gradient, against 64-bit arithmetic.
+    Bounds: a sum of `vocab` fp32 terms of one sign (1e-5 covers it), the ex2 approximation (2^-22)
+    and, for the fp16 gradient, one rounding of a value of at most 1024."""
+    from hackaton_b200.lm_loss import ce_grad, ce_stats
+
+    g = torch.Generator(device="cuda").manual_seed(rows + vocab)
+    logits = (torch.randn(rows, vocab, generator=g, device="cuda") * 3).to(dtype)
+    targets = torch.randint(0, vocab, (rows,), generator=g, device="cuda")
+    targets[::5] = -100
+    valid = targets >= 0
+    out = tuple(torch.empty(rows, device="cuda") for _ in range(3)) + (
+        torch.empty(rows, dtype=torch.int64, device="cuda"),)
+    ce_stats(logits, targets, True, out=out)
+    logp = torch.log_softmax(logits.double(), -1)
+    want = torch.logsumexp(logits.double(), -1)
+    picked = logp.gather(1, targets.clamp(min=0)[:, None])[:, 0]
+    close = lambda a, b, t: torch.testing.assert_close(a.double(), b, rtol=t, atol=t)  # noqa: E731
+    close(out[0][valid], want[valid], 1e-5)
+    close(out[1], torch.where(valid, -picked, 0.0), 2e-5)
+    close(out[2], -(logp.exp() * logp).sum(-1), 1e-4)
+    assert torch.equal(out[3], logits.argmax(-1)) or torch.equal(
+        logits.gather(1, out[3][:, None])[:, 0], logits.amax(-1))
+    grad = logp.exp()
+    grad.scatter_add_(1, targets.clamp(min=0)[:, None], torch.full_like(grad[:, :1], -1.0))
+    grad = torch.where(valid[:, None], grad * 1024, 0.0)
+    ce_grad(logits, targets, out[0], torch.full((1,), 1024.0, device="cuda"), logits)
+    close(logits, grad, 1e-3 if dtype == torch.float16 else 1e-3)
+    assert not logits[~valid].any()
+    cuda_lib.device_status()
+
+
+@pytest.mark.parametrize("rows", [2048, 2049, 2600])
+def test_chunks_cover_the_rows(cuda_lib, rows):
+    """Chunked against plain computation around the chunk limit (one chunk, two uneven ones)."""
+    from hackaton_b200.lm_loss import CHUNK_ROWS, _chunks, linear_cross_entropy
+
+    parts = _chunks(rows)
+    assert [p.start for p in parts] == [0] + [p.stop for p in parts[:-1]] and parts[-1].stop == rows
+    assert max(p.stop - p.start for p in parts) <= CHUNK_ROWS
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    hidden = (torch.randn(rows, 64, device="cuda", generator=g) * 0.5).half().requires_grad_()
+    weight = (torch.randn(1000, 64, device="cuda", generator=g) * 0.1).half()
+    targets = torch.randint(0, 1000, (rows,), device="cuda", generator=g)
+    denom = torch.tensor(float(rows), device="cuda")
+    logits = (hidden.detach().double() @ weight.double().t()).requires_grad_()
+    ref = torch.nn.functional.cross_entropy(logits, targets)
+    want = torch.autograd.grad(ref, logits)[0] @ weight.double()
+    loss, *_ = linear_cross_entropy(hidden, weight, targets, denom)
+    grad, = torch.autograd.grad(loss, hidden)
+    torch.testing.assert_close(loss.double(), ref, rtol=1e-4, atol=1e-4)
+    assert (grad.double() - want).norm() <= 5e-3 * want.norm()   # fp16 logits, gradients and sums
