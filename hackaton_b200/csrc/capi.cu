@@ -534,6 +534,8 @@ int64_t nf4b200_gate_up_swiglu_workspace_bytes(int64_t n_rows, int64_t n_cols, i
     if (n_rows <= 0 || n_cols <= 0 || m <= 0)
         return fail(NF4B200_EINVAL, "gate_up_swiglu_workspace_bytes: bad shape");
     if (m > 256) return 0;  // epilogue-fused kernel: no scratch
+    // (up to 64 rows the streaming kernel forms the product too, but only for weights that bring a
+    // scale table: the scratch covers a call without one)
     long long rows[2] = {n_rows, n_rows};
     const nf4::GemmPlan pl = nf4::plan_gemm_group(m, rows, 2, n_cols, false, gemm_sms(d));
     const size_t gemm_ws = (pl.ws_bytes + 255) / 256 * 256;
@@ -576,6 +578,12 @@ int nf4b200_gate_up_swiglu_fwd(const nf4b200_weight* gate_w, const nf4b200_weigh
         cudaError_t e = nf4::launch_gate_up_swiglu(ga, static_cast<__half*>(hidden), n, st, &why);
         if (e != cudaSuccess)
             return fail(NF4B200_ECUDA, "gate_up_swiglu: %s: %s", why, cudaGetErrorString(e));
+        return NF4B200_OK;
+    }
+    if (nf4::gemv_swiglu_eligible(ga)) {
+        cudaError_t e = nf4::launch_gemv_swiglu(ga, static_cast<__half*>(hidden), st);
+        if (e != cudaSuccess)
+            return fail(NF4B200_ECUDA, "gate_up_swiglu: small-M kernel: %s", cudaGetErrorString(e));
         return NF4B200_OK;
     }
     // few token rows: grouped GEMM, then the elementwise kernel; without gate_out / up_out the two

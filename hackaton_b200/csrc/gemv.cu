@@ -1,20 +1,28 @@
 // NF4 linear for a handful of token rows (the decode shapes of serving), both directions:
 //   forward  (M <= 64): out_i[M, N_i] = act[M, K] . W_i^T (+ bias_i) (+ ext_a_i . ext_b_i^T)
 //   backward (M <= 16): out[M, K]     = sum_i act_i[M, N_i] . W_i  (+ ext_a_i . ext_b_i)
-// for a group of up to four weights that share K (forward: they also share the activations).
+// for a group of up to four weights that share K (forward: they also share the activations; gate and
+// up can leave as silu(gate) * up).
 // At these sizes the work is reading the packed weights once (0.52 B per weight); a 128-row
 // tensor-core tile would be 50-99 % padding and the persistent tcgen05 kernel's set-up and
-// epilogue would dominate. So: no shared-memory ring, no TMEM. Warps stream the codes straight
-// from global memory, expand them in registers with the same byte-permute table look-up as the
-// big kernel (same rounding: fp16(table) * fp16(scale)) and multiply with warp-level mma.sync
-// (m16n8k16, fp32 accumulate). Forward with up to 8 token rows: a byte -> fp16-pair table in
-// shared memory instead, and the block scale applied to each k-block's fp32 sums.
+// epilogue would dominate. So: no TMEM. Warps bring the codes into private rings in shared memory,
+// expand them and multiply with warp-level mma.sync (m16n8k16, fp32 accumulate).
 //
-// Forward: a CTA owns 16 weight rows of one member of the group, its warps split the 64-deep
+// Forward: a warp owns 16 or 32 weight rows of one member of the group and a slice of the 64-deep
 // k-blocks. The contraction index is visited in a permuted order that A (weights) and B (tokens)
 // share, so a thread's 16 consecutive weights and 16 consecutive activations feed four k16 steps
-// without any shuffle. The warps' partial tiles are added through shared memory; bias and the
-// rank-16 LoRA term are applied there.
+// without any shuffle. A byte of codes is expanded by one look-up in a byte -> fp16-pair table, and
+// the block scale is applied to each k-block's fp32 sums (one rounding less than scaling weights).
+// The warps' partial tiles are added through shared memory; bias, the rank-16 LoRA term and the
+// SwiGLU product are applied there.
+// What bounds it: the L1 / shared-memory pipe (per 16 rows x 64 weights: 16 wavefronts of look-ups,
+// 8 of codes through the ring, 2 of scales, 2 to 32 of activations) and, with few k-blocks per warp,
+// the launch itself (1.65 us for an empty kernel in a chain). Measured in CUDA graphs over rotating
+// layers, us per layer (q/k/v, o, gate / up + product, down), before (codes loaded straight into
+// registers, table look-ups with bank conflicts or by byte permutes, product as a kernel of its own)
+// -> now: 1536-wide network, 1 row 28.9 -> 18.6, 16 rows 32.6 -> 25.2, 32 rows 51.8 -> 36.4;
+// 3584-wide, 1 row 87 -> 53, 16 rows 94.5 -> 66.7, 32 rows 125.6 -> 96.4. The weights alone
+// at the copy bandwidth: 3.7 and 18.4 us.
 //
 // Backward: the contraction runs over weight rows, along which the codes are NOT contiguous. A
 // warp owns one k-block (64 output columns) and a slab of weight rows; per step of 16 rows lane
@@ -42,15 +50,13 @@
 #include "decode.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
+#include "swiglu.cuh"
 
 namespace nf4 {
 
 constexpr int GV_ROWS = 16;
-#ifndef GV_BATCH_N
-#define GV_BATCH_N 4
-#endif
-constexpr int GV_BATCH = GV_BATCH_N;
 constexpr int GV_MAXP = GEMM_MAX_GROUP;
+constexpr int GV_MAX_SMEM = 227 * 1024;
 
 struct GemvProblem {
     const uint8_t* codes;
@@ -63,7 +69,8 @@ struct GemvProblem {
     __half* out;             // forward: this member's output
     long long ld_out, ld_act;
     int n_w;
-    int first;               // forward: first CTA of this member; backward: first row slab
+    int first;               // forward: first set of this member; backward: first row slab
+    int tiles;               // forward: tiles of this member
 };
 
 struct GemvParams {
@@ -73,15 +80,16 @@ struct GemvParams {
     float* planes;           // backward: [slabs][M][ldp] fp32
     long long ldp;
     int n_prob, m, k_w;
+    int split_log, n_sets;   // forward: log2(warps per tile), CTA-sized sets of tiles of the whole group
+    __half* hidden;          // forward with SwiGLU: the product
     int rows_per_slab;       // backward: weight rows per CTA (multiple of 16 * warps)
     int ticket_base;         // backward: first ticket of this launch, or -1 (reduction by a second kernel)
     int n_slabs;
-    int prefetch;            // codes are 16-byte aligned: bulk L2 prefetch is legal
 };
 
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                           uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -93,28 +101,27 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 __device__ __forceinline__ void mma_16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                                 uint32_t a3, uint32_t b0, uint32_t b1) {
     const float z = 0.f;
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(z));
 }
 
-__device__ __forceinline__ uint32_t gv_lds32(uint32_t addr) {
+// Forward decode by byte: a 256-entry table in shared memory maps a byte of codes to its two
+// unscaled fp16 table values (first weight = high nibble in the low half). It is kept once per
+// bank (lane l reads copy l), so a warp's 32 look-ups are one conflict-free wavefront. Where gate and
+// up are multiplied together their two tables share 256-byte entries.
+// The table sits at a fixed shared-memory address, so that the base is an immediate of the load:
+// behind the 1 KB that the system reserves at the start of a block's shared memory (the kernel
+// has no static shared memory, so its dynamic part starts right there).
+constexpr uint32_t PAIR_AT = 2048;
+
+__device__ __forceinline__ uint32_t pair_lookup(uint32_t offset) {
     uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+    asm("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(offset), "n"(PAIR_AT));
     return v;
 }
-
-// Forward decode by byte: a 256-entry table in shared memory maps a byte of codes to its two
-// unscaled fp16 table values (first weight = high nibble in the low half), kept in PAIR_COPIES
-// copies (lane l reads copy l % PAIR_COPIES) so that a warp's look-ups spread over the banks.
-// One look-up per two weights instead of 27 register instructions per eight; the block scale
-// is applied to the k-block's fp32 sums instead of to every weight (one rounding less). Used for
-// up to 8 token rows (one token block): measured at M = 1, each group timed alone, 26.2 -> 24.0 us
-// per layer forward, while with two token blocks (M = 16) the per-block scaling costs more than
-// the look-ups save (gate/up 14.8 -> 19.0 us), so those keep the register look-up.
-constexpr int PAIR_COPIES = 8;
 
 __device__ __forceinline__ RegLut load_reg_lut(const float* code16) {
     uint16_t bits[16];
@@ -141,172 +148,284 @@ __device__ __forceinline__ void prefetch_span(const uint8_t* ptr, long long byte
     }
 }
 
-// (the 4-warp instantiation for one token block is capped at 64 registers: eight CTAs per SM, so
-// the 1120 CTAs of a gate/up group are one wave)
-template <int NT, int GV_WARPS>  // token blocks of 8 (M <= 8 * NT); warps that split K
-__global__ void __launch_bounds__(GV_WARPS * 32, (GV_WARPS == 4 && NT == 1) ? 8 : 1)
+// Forward. A warp tile is MT * 16 weight rows of one member of the group (SWIGLU: the same 16 rows
+// of gate and of up) times up to 32 tokens; 2^split_log warps share a tile, each with a contiguous
+// slice of its k-blocks, and a CTA of 16 warps holds the other tiles of a set. Every warp brings its
+// own codes and scales through a private ring in shared memory (cp.async), laid out [k-block][row]
+// [32 bytes], from which its fragments (rows g, g + 8; 8 bytes each) are read without conflicts: a
+// direct load of such a fragment touches eight lines, which cost as much of the L1 pipe as the
+// look-ups.
+template <int NT, int MT, bool SWIGLU, int WL>
+struct GemvShape {
+    static constexpr int WARPS = 1 << WL, THREADS = WARPS * 32;
+    static constexpr int KBS = MT == 1 ? 4 : 2;        // k-blocks per ring stage
+    static constexpr int STAGES = NT == 1 && MT == 1 ? 3 : 2;
+    static constexpr int SLOT = 2048 + 128;            // codes and scales of a stage: MT * KBS * (512 + 32)
+    static constexpr int RING = STAGES * SLOT;         // per warp
+    static constexpr int ROWS = GV_ROWS * MT;
+    static constexpr int STRIDE = SWIGLU ? 256 : 128;  // bytes per table entry
+    static constexpr int TABLE_BYTES = 256 * STRIDE;
+    static constexpr int RED_BYTES = WARPS * NT * 8 * (ROWS + 1) * 4;   // takes the rings' place
+    static constexpr int RINGS_BYTES = WARPS * RING;
+    static constexpr int FIXED_BYTES = TABLE_BYTES + (RED_BYTES > RINGS_BYTES ? RED_BYTES : RINGS_BYTES);
+};
+
+// XS: the activations are staged in shared memory
+template <int NT, int MT, bool SWIGLU, bool XS, int WL>
+__global__ void __launch_bounds__(32 << WL, NT * MT == 1 || WL == 3 ? 2 : 1)
 nf4_gemv_kernel(const __grid_constant__ GemvParams p) {
-    constexpr int GV_THREADS = GV_WARPS * 32;
-    const int pi = gemv_find(p, (int)blockIdx.x);
-    const GemvProblem& pr = p.prob[pi];
-    const int r0 = ((int)blockIdx.x - pr.first) * GV_ROWS;
-    const size_t row_bytes = (size_t)p.k_w >> 1;
-    // The CTA's 16 rows of codes are one contiguous span: on its way to L2 while the previous
-    // kernel of the stream is still running.
-    if (threadIdx.x == 0 && p.prefetch)
-        prefetch_span(pr.codes + (size_t)r0 * row_bytes, (long long)(GV_ROWS * row_bytes));
-    grid_dep_wait();
-    grid_dep_launch();
-    __shared__ float red[GV_WARPS][NT * 8][GV_ROWS + 1];
-    constexpr bool PAIR = NT == 1;
-    __shared__ uint32_t pair_table[PAIR ? 256 * PAIR_COPIES : 1];
+    using Shape = GemvShape<NT, MT, SWIGLU, WL>;
+    constexpr int KBS = Shape::KBS, ROWS = Shape::ROWS, STAGES = Shape::STAGES;
+    static_assert(!SWIGLU || MT == 2, "gate and up rows are the two row blocks of a tile");
+    extern __shared__ __align__(256) uint8_t smem[];
+    uint8_t* const table = smem + (PAIR_AT - (uint32_t)__cvta_generic_to_shared(smem));
+    float (*red)[NT * 8][ROWS + 1] = reinterpret_cast<float (*)[NT * 8][ROWS + 1]>(table + Shape::TABLE_BYTES);
+    __half* xs = reinterpret_cast<__half*>(table + Shape::FIXED_BYTES);
+
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int r_lo = r0 + g, r_hi = r0 + g + 8;  // n_w % 16 == 0: both inside the weight
-
-    float acc[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-
+    const uint32_t row_bytes = (uint32_t)p.k_w >> 1;
     const int nkb = p.k_w >> 6;
-#ifdef GV_INTERLEAVE
-    // warps take the k-blocks in turn: at any moment the warps of a CTA read neighbouring 32-byte
-    // pieces of the same 128-byte lines
-    const int kb_begin = warp, kb_end = nkb;
-    constexpr int KB_STEP = GV_WARPS;
-#else
-    const int kb_begin = nkb * warp / GV_WARPS, kb_end = nkb * (warp + 1) / GV_WARPS;
-    constexpr int KB_STEP = 1;
-#endif
-    const uint8_t* c_lo = pr.codes + (size_t)r_lo * row_bytes + t * 8;
-    const uint8_t* c_hi = pr.codes + (size_t)r_hi * row_bytes + t * 8;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const int slots_log = WL - p.split_log, slots = 1 << slots_log;  // tiles of a set
+    const int slot = warp >> p.split_log, slice = warp & ((1 << p.split_log) - 1);
+    const int kb_begin = (nkb * slice) >> p.split_log, kb_end = (nkb * (slice + 1)) >> p.split_log;
 
-    // k-blocks in batches of GV_BATCH: all of a batch's code and scale loads are issued before the
-    // first one is used, so a warp pays the memory latency once per batch, not once per k-block.
-    // The first batch goes out before the table look-up is built, so that the table's own loads
-    // share its round trip instead of preceding it.
-    uint2 q_lo[GV_BATCH], q_hi[GV_BATCH];
-    __half s_lo[GV_BATCH], s_hi[GV_BATCH];
-    auto issue = [&](int kb0) {
+    // A set's tiles belong to one member (SWIGLU: to gate and up alike). Member of a set, weight of
+    // row block mt, first row of row block mt of a tile:
+    auto member_of = [&](int set) { return SWIGLU ? 0 : gemv_find(p, set); };
+    auto problem = [&](int pi, int mt) -> const GemvProblem& { return p.prob[SWIGLU ? mt : pi]; };
+    auto row_of = [&](int tile, int mt) { return SWIGLU ? tile * GV_ROWS : tile * ROWS + mt * GV_ROWS; };
+    // On their way to L2 while the previous kernel of the stream is still running: the rows of codes
+    // of a tile (one contiguous span) and its block scales (a 32-byte piece per k-block).
+    {
+        const int pi = member_of((int)blockIdx.x);
+        const int tile0 = ((int)blockIdx.x - problem(pi, 0).first) << slots_log;
+        const int valid = problem(pi, 0).tiles - tile0;
+        if ((int)threadIdx.x < slots * MT) {
+            const int sl = (int)threadIdx.x / MT, mt = (int)threadIdx.x % MT;
+            if (sl < valid)
+                prefetch_span(problem(pi, mt).codes + (size_t)row_of(tile0 + sl, mt) * row_bytes,
+                              (long long)GV_ROWS * row_bytes);
+        }
+        if (slot < valid) {
 #pragma unroll
-        for (int b = 0; b < GV_BATCH; ++b) {
-            const int kb = min(kb0 + b * KB_STEP, kb_end - 1);  // (tail: re-reads the last block, unused)
-            // this thread's 16 weights of rows r_lo and r_hi: k = kb*64 + 16t .. + 15
-            q_lo[b] = __ldg(reinterpret_cast<const uint2*>(c_lo + (size_t)kb * 32));
-            q_hi[b] = __ldg(reinterpret_cast<const uint2*>(c_hi + (size_t)kb * 32));
-            s_lo[b] = __ldg(pr.scales16 + (size_t)kb * pr.n_w + r_lo);
-            s_hi[b] = __ldg(pr.scales16 + (size_t)kb * pr.n_w + r_hi);
+            for (int mt = 0; mt < MT; ++mt) {
+                const GemvProblem& pr = problem(pi, mt);
+                for (int kb = kb_begin + lane; kb < kb_end; kb += 32)
+                    prefetch_l2(pr.scales16 + (size_t)kb * pr.n_w + row_of(tile0 + slot, mt));
+            }
         }
-    };
-    if (kb_begin < kb_end) issue(kb_begin);
-    RegLut lut = {};
-    uint32_t pair_base = 0;
-    if constexpr (PAIR) {
-        // (red is free until the fold: it holds the 16 fp16 table values while the pairs are built)
-        unsigned short* t16 = reinterpret_cast<unsigned short*>(&red[0][0][0]);
-        if (threadIdx.x < 16)
-            t16[threadIdx.x] = __half_as_ushort(__float2half_rn(__ldg(pr.code16 + threadIdx.x)));
-        __syncthreads();
-        for (int i = threadIdx.x; i < 256 * PAIR_COPIES; i += GV_THREADS) {
-            const int e = i / PAIR_COPIES;
-            pair_table[i] = (uint32_t)t16[e >> 4] | ((uint32_t)t16[e & 15] << 16);
-        }
-        __syncthreads();
-        pair_base = (uint32_t)__cvta_generic_to_shared(pair_table) + (lane % PAIR_COPIES) * 4;
-    } else {
-        lut = load_reg_lut(pr.code16);
     }
-    auto pairs = [&](uint32_t w, uint32_t (&o)[8], int at) {
+    grid_dep_wait();
+    grid_dep_launch();
+
+    // the tokens of this CTA (blockIdx.y: blocks of NT * 8)
+    const int token0 = (int)blockIdx.y * NT * 8, tokens = min(p.m - token0, NT * 8);
+    const __half* const act = p.act + token0 * p.ld_act;
+    const uint32_t lane4 = lane * 4;
+    auto pairs = [&](int mt, uint32_t w, uint32_t (&o)[8], int at) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            o[at + i] = gv_lds32(pair_base + ((w >> (8 * i)) & 0xFFu) * (4u * PAIR_COPIES));
+            o[at + i] = pair_lookup(SWIGLU ? __byte_perm(w, lane4 + mt * 128, 0x7604u + (i << 4))
+                                           : __byte_perm(w, 0u, 0x4440u + i) * 128u + lane4);
     };
+    const uint32_t ring = PAIR_AT + Shape::TABLE_BYTES + warp * Shape::RING;   // shared-memory address
+    const uint8_t* const ring_ptr = table + Shape::TABLE_BYTES + warp * Shape::RING;
 
-    for (int kb0 = kb_begin; kb0 < kb_end; kb0 += GV_BATCH * KB_STEP) {
-        if (kb0 != kb_begin) issue(kb0);
+    int built = -1;   // the member whose pair table is in place
+    for (int set = (int)blockIdx.x; set < p.n_sets; set += (int)gridDim.x) {
+        const int pi = member_of(set);
+        const int tile0 = (set - problem(pi, 0).first) << slots_log, tile = tile0 + slot;
+        const bool build = pi != built;
+        // the two table values of this thread's table entry: their loads share the first round trip
+        constexpr int ENTRIES = 512 / Shape::THREADS;   // table entries (halves of, where SWIGLU) per thread
+        const GemvProblem& tp = problem(pi, SWIGLU ? (threadIdx.x & 1) : 0);
+        float code_hi[ENTRIES], code_lo[ENTRIES];
+        if (build) {
 #pragma unroll
-        for (int b = 0; b < GV_BATCH; ++b) {
-            const int kb = kb0 + b * KB_STEP;
-            if (kb >= kb_end) break;
-            uint32_t wl[8], wh[8];
-            const float f_lo = __half2float(s_lo[b]), f_hi = __half2float(s_hi[b]);
-            if constexpr (PAIR) {
-                pairs(q_lo[b].x, wl, 0); pairs(q_lo[b].y, wl, 4);
-                pairs(q_hi[b].x, wh, 0); pairs(q_hi[b].y, wh, 4);
-            } else {
-                const uint4 a = decode_word_reg(q_lo[b].x, lut, __half2half2(s_lo[b]));
-                const uint4 c = decode_word_reg(q_lo[b].y, lut, __half2half2(s_lo[b]));
-                wl[0] = a.x; wl[1] = a.y; wl[2] = a.z; wl[3] = a.w;
-                wl[4] = c.x; wl[5] = c.y; wl[6] = c.z; wl[7] = c.w;
-                const uint4 d = decode_word_reg(q_hi[b].x, lut, __half2half2(s_hi[b]));
-                const uint4 e = decode_word_reg(q_hi[b].y, lut, __half2half2(s_hi[b]));
-                wh[0] = d.x; wh[1] = d.y; wh[2] = d.z; wh[3] = d.w;
-                wh[4] = e.x; wh[5] = e.y; wh[6] = e.z; wh[7] = e.w;
+            for (int i = 0; i < ENTRIES; ++i) {
+                const int entry = (threadIdx.x + i * Shape::THREADS) >> 1;
+                code_hi[i] = __ldg(tp.code16 + (entry >> 4));
+                code_lo[i] = __ldg(tp.code16 + (entry & 15));
             }
-            const long long kcol = (long long)kb * 64 + t * 16;
+        }
+        if (XS && set == (int)blockIdx.x) {   // staged once, read by every warp
+            const int chunks = p.k_w / 8;
+            for (int token = 0; token < tokens; ++token) {
+                const __half* src = act + (long long)token * p.ld_act;
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs) + token * (p.k_w + 8) * 2;
+                for (int c = threadIdx.x; c < chunks; c += Shape::THREADS) cp_async16(dst + c * 16, src + c * 8);
+            }
+        }
+        cp_async_commit();
+
+        const int count = tile < problem(pi, 0).tiles ? kb_end - kb_begin : 0;
+        // Ring stage: lane = (row, 16-byte chunk) of KBS k-blocks (byte offsets: a member's codes are
+        // below 4 GB); the first 8 lanes bring the scales, 16 bytes each.
+        constexpr int CHUNKS = KBS * 2, ROWS_PER = 32 / CHUNKS;
+        const int c_row = lane / CHUNKS, c_at = lane % CHUNKS;
+        const uint32_t c_dst = (c_at >> 1) * 512 + c_row * 32 + (c_at & 1) * 16;
+        const uint8_t* c_src[MT];
+        uint32_t c_off[MT];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            c_src[mt] = problem(pi, mt).codes;
+            c_off[mt] = (uint32_t)(row_of(tile, mt) + c_row) * row_bytes + kb_begin * 32 + c_at * 16;
+        }
+        const int s_mt = lane / CHUNKS, s_kb = c_at >> 1;   // lanes 0 .. CHUNKS * MT - 1 = 0 .. 7
+        const GemvProblem& sp = problem(pi, s_mt < MT ? s_mt : 0);
+        const uint8_t* const s_src = reinterpret_cast<const uint8_t*>(
+            sp.scales16 + (size_t)(kb_begin + s_kb) * sp.n_w + row_of(tile, s_mt)) + (c_at & 1) * 16;
+        const uint32_t s_step = 2 * (uint32_t)sp.n_w;
+        auto fill = [&](int i0, uint32_t at) {   // k-blocks i0 .. i0 + KBS - 1 of the slice
+            if (i0 + (c_at >> 1) < count) {
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int r = 0; r < GV_ROWS / ROWS_PER; ++r)
+                        cp_async16(at + mt * (KBS * 512) + c_dst + r * (ROWS_PER * 32),
+                                   c_src[mt] + (c_off[mt] + i0 * 32 + r * ROWS_PER * row_bytes));
+                if (lane < CHUNKS * MT)
+                    cp_async16(at + 2048 + s_mt * (KBS * 32) + s_kb * 32 + (c_at & 1) * 16,
+                               s_src + (size_t)i0 * s_step);
+            }
+            cp_async_commit();
+        };
+#pragma unroll
+        for (int st = 0; st < STAGES - 1; ++st) fill(st * KBS, ring + st * Shape::SLOT);
+
+        if (build) {
+            // the 32 copies of an entry: by one thread per table, or half of them by each of the two;
+            // 16-byte stores rotated over the banks
+#pragma unroll
+            for (int i = 0; i < ENTRIES; ++i) {
+                const int entry = (threadIdx.x + i * Shape::THREADS) >> 1;
+                const uint32_t pair = (uint32_t)__half_as_ushort(__float2half_rn(code_hi[i])) |
+                                      ((uint32_t)__half_as_ushort(__float2half_rn(code_lo[i])) << 16);
+                const uint4 v = make_uint4(pair, pair, pair, pair);
+                uint4* dst = reinterpret_cast<uint4*>(table + entry * Shape::STRIDE) + (SWIGLU ? (threadIdx.x & 1) * 8 : 0);
+                constexpr int STORES = SWIGLU ? 8 : 4;
+                const int at = SWIGLU ? 0 : (threadIdx.x & 1) * 4;
+#pragma unroll
+                for (int j = 0; j < STORES; ++j) dst[at + ((j + entry) & (STORES - 1))] = v;
+            }
+            built = pi;
+        }
+        float acc[MT][NT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+                acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.f;
+        // Token nt * 8 + g, this thread's 16 columns of a k-block (tokens past the last one read the
+        // last one's row again: their sums are not written).
+        const long long x_ld = XS ? p.k_w + 8 : p.ld_act;
+        const __half* x_at[NT];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+            x_at[nt] = (XS ? xs : act) + min(nt * 8 + g, tokens - 1) * x_ld + kb_begin * 64 + t * 16;
+        cp_async_wait<STAGES - 1>();   // the staged activations
+        __syncthreads();
+
+        int read = 0, write = STAGES - 1;   // ring stages
+        for (int i0 = 0; i0 < count; i0 += KBS) {
+            cp_async_wait<STAGES - 2>();
+            __syncwarp();      // the stage has landed for all lanes, and all have left the one before it
+            fill(i0 + (STAGES - 1) * KBS, ring + write * Shape::SLOT);
+            const uint8_t* const st = ring_ptr + read * Shape::SLOT;
+            write = write + 1 == STAGES ? 0 : write + 1;
+            read = read + 1 == STAGES ? 0 : read + 1;
+#pragma unroll
+            for (int j = 0; j < KBS; ++j) {
+                if (i0 + j >= count) break;
+                uint32_t wl[MT][8], wh[MT][8];
+                float f_lo[MT], f_hi[MT];
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    const uint8_t* c = st + (mt * KBS + j) * 512 + g * 32 + t * 8;
+                    const uint2 lo = *reinterpret_cast<const uint2*>(c);
+                    const uint2 hi = *reinterpret_cast<const uint2*>(c + 256);
+                    const __half* sc = reinterpret_cast<const __half*>(st + 2048 + (mt * KBS + j) * 32) + g;
+                    f_lo[mt] = __half2float(sc[0]);
+                    f_hi[mt] = __half2float(sc[8]);
+                    pairs(mt, lo.x, wl[mt], 0); pairs(mt, lo.y, wl[mt], 4);
+                    pairs(mt, hi.x, wh[mt], 0); pairs(mt, hi.y, wh[mt], 4);
+                }
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    // the same 16 k of the token: k16 step j takes words 2j, 2j+1 of both operands
+                    const uint4* xp = reinterpret_cast<const uint4*>(x_at[nt] + (i0 + j) * 64);
+                    const uint4 x0 = xp[0], x1 = xp[1];
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        // unscaled sums of this k-block, then the rows' block scales (d0, d1: row g;
+                        // d2, d3: row g + 8)
+                        float blk[4];
+                        mma_16816_first(blk, wl[mt][0], wh[mt][0], wl[mt][1], wh[mt][1], x0.x, x0.y);
+                        mma_16816(blk, wl[mt][2], wh[mt][2], wl[mt][3], wh[mt][3], x0.z, x0.w);
+                        mma_16816(blk, wl[mt][4], wh[mt][4], wl[mt][5], wh[mt][5], x1.x, x1.y);
+                        mma_16816(blk, wl[mt][6], wh[mt][6], wl[mt][7], wh[mt][7], x1.z, x1.w);
+                        acc[mt][nt][0] = fmaf(f_lo[mt], blk[0], acc[mt][nt][0]);
+                        acc[mt][nt][1] = fmaf(f_lo[mt], blk[1], acc[mt][nt][1]);
+                        acc[mt][nt][2] = fmaf(f_hi[mt], blk[2], acc[mt][nt][2]);
+                        acc[mt][nt][3] = fmaf(f_hi[mt], blk[3], acc[mt][nt][3]);
+                    }
+                }
+            }
+        }
+        cp_async_wait<0>();
+        __syncthreads();   // the rings are idle: their place is the fold's
+        // accumulator fragment: d0,d1 -> (weight row g, tokens 2t, 2t+1); d2,d3 -> (row g+8, same)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                // the same 16 k of token nt*8 + g: k16 step j takes words 2j, 2j+1 of both operands
-                const int token = nt * 8 + g;
-                uint4 x0 = zero, x1 = zero;
-                if (token < p.m) {
-                    const uint4* xp =
-                        reinterpret_cast<const uint4*>(p.act + (long long)token * p.ld_act + kcol);
-                    x0 = __ldg(xp);
-                    x1 = __ldg(xp + 1);
-                }
-                if constexpr (PAIR) {
-                // unscaled sums of this k-block, then the rows' block scales (d0, d1: row g; d2, d3: g + 8)
-                float blk[4];
-                mma_16816_first(blk, wl[0], wh[0], wl[1], wh[1], x0.x, x0.y);
-                mma_16816(blk, wl[2], wh[2], wl[3], wh[3], x0.z, x0.w);
-                mma_16816(blk, wl[4], wh[4], wl[5], wh[5], x1.x, x1.y);
-                mma_16816(blk, wl[6], wh[6], wl[7], wh[7], x1.z, x1.w);
-                acc[nt][0] = fmaf(f_lo, blk[0], acc[nt][0]);
-                acc[nt][1] = fmaf(f_lo, blk[1], acc[nt][1]);
-                acc[nt][2] = fmaf(f_hi, blk[2], acc[nt][2]);
-                acc[nt][3] = fmaf(f_hi, blk[3], acc[nt][3]);
-                } else {
-                mma_16816(acc[nt], wl[0], wh[0], wl[1], wh[1], x0.x, x0.y);
-                mma_16816(acc[nt], wl[2], wh[2], wl[3], wh[3], x0.z, x0.w);
-                mma_16816(acc[nt], wl[4], wh[4], wl[5], wh[5], x1.x, x1.y);
-                mma_16816(acc[nt], wl[6], wh[6], wl[7], wh[7], x1.z, x1.w);
-                }
+                red[warp][nt * 8 + 2 * t][mt * 16 + g] = acc[mt][nt][0];
+                red[warp][nt * 8 + 2 * t + 1][mt * 16 + g] = acc[mt][nt][1];
+                red[warp][nt * 8 + 2 * t][mt * 16 + g + 8] = acc[mt][nt][2];
+                red[warp][nt * 8 + 2 * t + 1][mt * 16 + g + 8] = acc[mt][nt][3];
             }
-        }
-    }
-    __syncthreads();   // (the pair table build used `red`; every warp is past its look-ups)
-
-    // accumulator fragment: d0,d1 -> (weight row g, tokens 2t, 2t+1); d2,d3 -> (row g+8, same)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        red[warp][nt * 8 + 2 * t][g] = acc[nt][0];
-        red[warp][nt * 8 + 2 * t + 1][g] = acc[nt][1];
-        red[warp][nt * 8 + 2 * t][g + 8] = acc[nt][2];
-        red[warp][nt * 8 + 2 * t + 1][g + 8] = acc[nt][3];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < NT * 8 * GV_ROWS; e += GV_THREADS) {
-        const int token = e / GV_ROWS, r = e % GV_ROWS;  // 16 consecutive rows: 32 bytes of out
-        if (token >= p.m) continue;
-        float v = 0.f;
-#pragma unroll
-        for (int w = 0; w < GV_WARPS; ++w) v += red[w][token][r];
-        if (pr.ext_a != nullptr) {
-            const __half2* xa = reinterpret_cast<const __half2*>(pr.ext_a + (long long)token * 16);
-            const __half2* lb = reinterpret_cast<const __half2*>(pr.ext_b + (long long)(r0 + r) * 16);
-            float s = 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float2 a = __half22float2(__ldg(xa + j)), b = __half22float2(__ldg(lb + j));
-                s = fmaf(a.x, b.x, s);
-                s = fmaf(a.y, b.y, s);
+        __syncthreads();
+        constexpr int OUT_ROWS = SWIGLU ? GV_ROWS : ROWS;   // a power of two, like the slots
+        const GemvProblem& pr = problem(pi, 0);
+        for (int e = threadIdx.x; e < (tokens * OUT_ROWS) << slots_log; e += Shape::THREADS) {
+            const int r = e % OUT_ROWS, sl = (e / OUT_ROWS) & (slots - 1), tok = (e / OUT_ROWS) >> slots_log;
+            const int token = token0 + tok, w0 = sl << p.split_log;
+            if (tile0 + sl >= pr.tiles) continue;
+            float v = 0.f, u = 0.f;
+#pragma unroll 4
+            for (int w = 0; w < (1 << p.split_log); ++w) {
+                v += red[w0 + w][tok][r];
+                if (SWIGLU) u += red[w0 + w][tok][(GV_ROWS + r) % ROWS];
             }
-            v += s;
+            const int row = row_of(tile0 + sl, 0) + r;
+            if (SWIGLU) {
+                const __half hg = __float2half_rn(v), hu = __float2half_rn(u);
+                const long long at = (long long)token * pr.ld_out + row;
+                if (pr.out != nullptr) {
+                    pr.out[at] = hg;
+                    p.prob[1].out[at] = hu;
+                }
+                const float gf = __half2float(hg);
+                p.hidden[at] = __float2half_rn(gf * sigmoid_fast(gf) * __half2float(hu));
+                continue;
+            }
+            if (pr.ext_a != nullptr) {
+                const __half2* xa = reinterpret_cast<const __half2*>(pr.ext_a + (long long)token * 16);
+                const __half2* lb = reinterpret_cast<const __half2*>(pr.ext_b + (long long)row * 16);
+                float s = 0.f;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float2 a = __half22float2(__ldg(xa + j)), b = __half22float2(__ldg(lb + j));
+                    s = fmaf(a.x, b.x, s);
+                    s = fmaf(a.y, b.y, s);
+                }
+                v += s;
+            }
+            if (pr.bias != nullptr) v += __half2float(__ldg(pr.bias + row));
+            pr.out[(long long)token * pr.ld_out + row] = __float2half_rn(v);
         }
-        if (pr.bias != nullptr) v += __half2float(__ldg(pr.bias + r0 + r));
-        pr.out[(long long)token * pr.ld_out + r0 + r] = __float2half_rn(v);
+        if (set + (int)gridDim.x < p.n_sets) __syncthreads();   // `red` is free again
     }
 }
 
@@ -451,14 +570,16 @@ nf4_gemv_bwd_kernel(const __grid_constant__ GemvParams p) {
 
 static bool gemv_common_ok(const GemmArgs& a) {
     return a.scales16 != nullptr && a.n_w % GV_ROWS == 0 && a.k_w % 64 == 0 &&
-           (reinterpret_cast<uintptr_t>(a.codes) & 7) == 0;
+           (reinterpret_cast<uintptr_t>(a.codes) & 15) == 0;
 }
 
 bool gemv_eligible(const GemmArgs& a) {
-    // measured against the tensor-core kernel: always ahead up to 16 rows; up to 64 rows only for
-    // the small projections (the activations are re-read through L1/L2 once per 16 weight rows)
-    const bool small_enough = a.m <= 16 || (a.m <= 64 && a.n_w * a.k_w <= (1ll << 22));
-    return !a.trans_w && a.m >= 1 && small_enough && gemv_common_ok(a) && a.ld_act % 8 == 0 &&
+    // Measured against the tensor-core kernel: ahead up to 32 rows (four launches of a layer of the
+    // 1536-wide network 36 against 52 us, of the 3584-wide one 96 against 126); up to 64 rows, as two
+    // blocks of 32 tokens side by side, only where one block leaves SMs idle (64 rows, q/k/v of the
+    // 1536-wide one 6.3 against 15.6; its gate / up 26 against 24).
+    const bool small_enough = a.m <= 32 || (a.m <= 64 && a.n_w * a.k_w <= (1ll << 22));
+    return !a.trans_w && a.m >= 1 && small_enough && gemv_common_ok(a) && a.n_w * (a.k_w / 2) < (1ll << 32) && a.ld_act % 8 == 0 &&
            (reinterpret_cast<uintptr_t>(a.act) & 15) == 0;
 }
 
@@ -474,52 +595,117 @@ static void fill_problem(GemvProblem& q, const GemmArgs& a) {
     q.ld_out = a.ld_out; q.ld_act = a.ld_act; q.n_w = (int)a.n_w; q.first = 0;
 }
 
-template <int NT, int WARPS>
-static cudaError_t launch_gemv_t(const GemvParams& p, unsigned ctas, cudaStream_t stream) {
-    return launch_pdl(nf4_gemv_kernel<NT, WARPS>, dim3(ctas), dim3(WARPS * 32), 0, stream, p);
+template <int NT, int MT, bool SWIGLU, bool XS, int WL>
+static cudaError_t launch_gemv_x(const GemvParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
+    // the opt-in to more than 48 KB is a property of the kernel on a device: set once on each
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(done.load(std::memory_order_acquire) & bit)) {
+        e = cudaFuncSetAttribute(nf4_gemv_kernel<NT, MT, SWIGLU, XS, WL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 XS ? GV_MAX_SMEM : GemvShape<NT, MT, SWIGLU, WL>::FIXED_BYTES + (int)PAIR_AT);
+        if (e != cudaSuccess) return e;
+        done.fetch_or(bit, std::memory_order_release);
+    }
+    return launch_pdl(nf4_gemv_kernel<NT, MT, SWIGLU, XS, WL>, grid, dim3(32 << WL), smem, stream, p);
 }
 
-cudaError_t launch_gemv_group(const GemmGroupArgs& ga, cudaStream_t stream) {
+template <int NT, int MT, bool SWIGLU, int WL>
+static cudaError_t launch_gemv_t(GemvParams p, int sms, cudaStream_t stream) {
+    // Warps per tile: the fewest rounds of the busiest SM, then the fewest CTAs (the other half of
+    // an SM's registers is where the next kernel of the stream sets itself up).
+    const int nkb = p.k_w / 64, members = SWIGLU ? 1 : p.n_prob;
+    auto sets_of = [&](int i, int sl) { return (((long long)p.prob[i].tiles << sl) + (1 << WL) - 1) / (1 << WL); };
+    long long best = -1;
+    for (int sl = 0; sl <= WL && (sl == 0 || (1 << sl) <= nkb); ++sl) {
+        long long sets = 0;
+        for (int i = 0; i < members; ++i) sets += sets_of(i, sl);
+        const long long cost = (sets + sms - 1) / sms * ((1 << WL) >> sl);
+        if (best < 0 || cost < best) {
+            best = cost;
+            p.split_log = sl;
+            p.n_sets = (int)sets;
+        }
+    }
+    int first = 0;
+    for (int i = 0; i < members; ++i) {
+        p.prob[i].first = first;
+        first += (int)sets_of(i, p.split_log);
+    }
+    const dim3 grid((unsigned)(p.n_sets < 2 * sms ? p.n_sets : 2 * sms),
+                    (unsigned)((p.m + NT * 8 - 1) / (NT * 8)));
+    const size_t fixed = GemvShape<NT, MT, SWIGLU, WL>::FIXED_BYTES + PAIR_AT;
+    if constexpr (NT == 1) {
+        // Activations are staged (padded rows: 16-byte reads of eight rows meet no bank conflict) where
+        // that is one row or several tiles of the CTA read them, and read through L1 otherwise. us:
+        // one row, down_proj of 8960 columns 6.2 against 6.7; four rows, gate / up of the 3584-wide
+        // network (8 tiles) 25.0 against 28.6, its q/k/v (2 tiles) 6.6 against 6.4. With more than
+        // eight rows there was no gain.
+        const size_t x_bytes = (size_t)p.m * (p.k_w + 8) * 2;
+        if ((p.m == 1 || p.split_log <= WL - 2) && fixed + x_bytes <= (size_t)GV_MAX_SMEM)
+            return launch_gemv_x<NT, MT, SWIGLU, true, WL>(p, grid, fixed + x_bytes, stream);
+    }
+    return launch_gemv_x<NT, MT, SWIGLU, false, WL>(p, grid, fixed, stream);
+}
+
+template <int MT, bool SWIGLU>
+static cudaError_t launch_gemv_m(const GemvParams& p, int sms, cudaStream_t stream) {
+    if (p.m <= 8) return launch_gemv_t<1, MT, SWIGLU, 4>(p, sms, stream);
+    if (p.m <= 16) return launch_gemv_t<2, MT, SWIGLU, 4>(p, sms, stream);
+    if (p.m <= 32) return launch_gemv_t<4, MT, SWIGLU, 4>(p, sms, stream);
+    // two blocks of 32 tokens side by side: CTAs of 8 warps, two of which fit an SM
+    if constexpr (MT == 1 && !SWIGLU) return launch_gemv_t<4, 1, false, 3>(p, sms, stream);
+    return cudaErrorInvalidValue;
+}
+
+// Fills the parameters of a forward launch; `rows` = weight rows of a tile that come from one
+// member.
+static GemvParams gemv_forward_params(const GemmGroupArgs& ga, int rows) {
     const GemmArgs& a = ga.item[0];
     GemvParams p = {};
     p.n_prob = ga.count;
     p.act = a.act; p.ld_act = a.ld_act;
     p.m = (int)a.m; p.k_w = (int)a.k_w;
-    p.prefetch = 1;
-    long long ctas = 0;
     for (int i = 0; i < ga.count; ++i) {
         fill_problem(p.prob[i], ga.item[i]);
-        p.prob[i].first = (int)ctas;
-        ctas += ga.item[i].n_w / GV_ROWS;
-        if ((reinterpret_cast<uintptr_t>(ga.item[i].codes) & 15) != 0 || ((a.k_w / 2) * GV_ROWS) % 16 != 0)
-            p.prefetch = 0;
+        p.prob[i].tiles = (int)(ga.item[i].n_w / rows);
     }
     for (int i = ga.count; i < GV_MAXP; ++i) p.prob[i] = p.prob[0];
-    // Warps per CTA: with many row groups, small CTAs so that all of them are resident at once
-    // (a second round of CTAs costs as much as the first); with few row groups and long rows,
-    // 16 warps to spread K.
-    const int sms = a.sm_count > 0 ? a.sm_count : 148;
-    const int warps = ctas >= 3ll * sms ? 4 : (a.k_w >= 4096 && ctas < 2ll * sms ? 16 : 8);
-    const unsigned grid = (unsigned)ctas;
-    if (a.m <= 8) {
-        if (warps == 4) return launch_gemv_t<1, 4>(p, grid, stream);
-        if (warps == 16) return launch_gemv_t<1, 16>(p, grid, stream);
-        return launch_gemv_t<1, 8>(p, grid, stream);
-    }
-    if (a.m <= 16) {
-        if (warps == 4) return launch_gemv_t<2, 4>(p, grid, stream);
-        if (warps == 16) return launch_gemv_t<2, 16>(p, grid, stream);
-        return launch_gemv_t<2, 8>(p, grid, stream);
-    }
-    if (a.m <= 32) return launch_gemv_t<4, 8>(p, grid, stream);
-    return launch_gemv_t<8, 8>(p, grid, stream);
+    return p;
 }
 
-cudaError_t launch_gemv(const GemmArgs& a, cudaStream_t stream) {
-    GemmGroupArgs ga;
-    ga.count = 1;
-    ga.item[0] = a;
-    return launch_gemv_group(ga, stream);
+cudaError_t launch_gemv_group(const GemmGroupArgs& ga, cudaStream_t stream) {
+    const GemmArgs& a = ga.item[0];
+    const int sms = a.sm_count > 0 ? a.sm_count : 148;
+    // Tiles of 32 rows read the activations half as often: they pay with more than 8 tokens where they
+    // still occupy most SMs (us at 16 tokens, 32 against 16 rows: down_proj 3584 x 18944 21.7 against
+    // 26.9, 1536 x 8960 12.2 against 8.6).
+    long long rows = 0;
+    bool wide = a.m > 8 && a.m <= 32;
+    for (int i = 0; i < ga.count; ++i) {
+        wide = wide && ga.item[i].n_w % 32 == 0;
+        rows += ga.item[i].n_w;
+    }
+    if (rows / 32 * 4 < 3ll * sms) wide = false;
+    if (wide) return launch_gemv_m<2, false>(gemv_forward_params(ga, 2 * GV_ROWS), sms, stream);
+    return launch_gemv_m<1, false>(gemv_forward_params(ga, GV_ROWS), sms, stream);
+}
+
+bool gemv_swiglu_eligible(const GemmGroupArgs& ga) {
+    if (ga.count != 2) return false;
+    const GemmArgs &g = ga.item[0], &u = ga.item[1];
+    return g.m <= 32 && g.n_w == u.n_w && g.k_w == u.k_w && g.bias == nullptr && u.bias == nullptr &&
+           g.ext_a == nullptr && u.ext_a == nullptr && (g.out == nullptr) == (u.out == nullptr) &&
+           gemv_eligible(g) && gemv_eligible(u);
+}
+
+cudaError_t launch_gemv_swiglu(const GemmGroupArgs& ga, __half* hidden, cudaStream_t stream) {
+    const int sms = ga.item[0].sm_count > 0 ? ga.item[0].sm_count : 148;
+    GemvParams p = gemv_forward_params(ga, GV_ROWS);
+    p.hidden = hidden;
+    return launch_gemv_m<2, true>(p, sms, stream);
 }
 
 // Row slabs of the streaming backward: enough CTAs (k-blocks x slabs) for about three per SM, slabs

@@ -208,8 +208,11 @@ cudaError_t launch_ce(const CeArgs& a, cudaStream_t stream);
 // calls to them: forward for M <= 64 (a whole group in one launch), backward for M <= 16.
 bool gemv_eligible(const GemmArgs& a);
 bool gemv_bwd_eligible(const GemmArgs& a);
-cudaError_t launch_gemv(const GemmArgs& a, cudaStream_t stream);
 cudaError_t launch_gemv_group(const GemmGroupArgs& ga, cudaStream_t stream);
+// gate / up pair (item[0], item[1]) with hidden = silu(gate) * up formed where the rows' sums meet;
+// the items' `out` (row pitch as `hidden`) may both be null.
+bool gemv_swiglu_eligible(const GemmGroupArgs& ga);
+cudaError_t launch_gemv_swiglu(const GemmGroupArgs& ga, __half* hidden, cudaStream_t stream);
 cudaError_t launch_gemv_bwd_group(const GemmGroupArgs& ga, cudaStream_t stream, const char** why);
 // Row slabs of the streaming backward and the fp32 planes they need as scratch.
 struct StreamBwdPlan {

@@ -132,6 +132,24 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, i
                  : "memory");
 }
 
+// The line that holds `gptr`, brought into L2 (no values read, so nothing to order).
+__device__ __forceinline__ void prefetch_l2(const void* gptr) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(gptr));
+}
+
+// 16 bytes global -> shared without passing through registers, in groups: cp_async_wait<N> waits
+// until at most N of this thread's latest groups are still under way.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Asks for `bytes` (multiple of 16) at a 16-byte aligned global address to be brought into L2.
 __device__ __forceinline__ void bulk_prefetch_l2(const void* gptr, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gptr), "r"(bytes) : "memory");

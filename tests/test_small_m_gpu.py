@@ -181,3 +181,62 @@ def test_small_m_group_with_lora(cuda_lib, m):
         assert nf4_oracle.max_rel_err(y.detach().cpu(), want) <= TOL
     assert nf4_oracle.max_rel_err(xg.grad.cpu(), dx_ref) <= TOL
     assert cuda_lib.device_status() == 0
+
+
+def _odd_tables(state, seed):
+    """The same codes under another 16-entry table (tables are inputs of the kernels)."""
+    g = torch.Generator().manual_seed(seed)
+    state.code = (torch.rand(16, generator=g) * 2 - 1).cuda()
+    return state
+
+
+@pytest.mark.parametrize("m", [1, 2, 8, 9, 16, 17, 32, 33, 64])    # edges of the token blocks of 8, 16, 32
+@pytest.mark.parametrize("k", [64, 192, 1536, 8960])               # fewer k-blocks than warps, ragged slices
+def test_streaming_forward_every_plan(cuda_lib, m, k):
+    """Groups whose members differ in size and table, rows that are no multiple of 32, one weight
+    with enough rows for 32-row tiles, and gate / up with the product (with and without keeping
+    both), against the fp32 product of the bit-exact standalone decode. Bound: fp16 inputs and
+    outputs (2^-11 relative to the largest result) with fp32 sums of k terms; 2e-3 of the largest
+    element, as elsewhere in this file. Two calls give the same bits."""
+    from hackaton_b200.group import linear_forward_group
+    from hackaton_b200.mlp import gate_up_swiglu_forward
+    from hackaton_b200.nf4 import dequantize_nf4
+
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    x = torch.randn(m, k, generator=g, device="cuda").half()
+    rows = ((16, 48, 272), (3552,)) if k < 8960 else ((16, 48, 272), (1536,))
+    for group in rows:
+        weights = [synthetic_weight(n, k, True, seed=n + m, device="cuda") for n in group]
+        weights = [(p, _odd_tables(s, i)) if i else (p, s) for i, (p, s) in enumerate(weights)]
+        ys, again = linear_forward_group(x, weights), linear_forward_group(x, weights)
+        for y, y2, (p, s) in zip(ys, again, weights):
+            want = x.float() @ dequantize_nf4(p, s).float().t()
+            assert float((y.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+            assert torch.equal(y, y2)
+    n = 304
+    gate, up = (synthetic_weight(n, k, True, seed=7 * i + m, device="cuda") for i in (1, 2))
+    up = (up[0], _odd_tables(up[1], 5))
+    hidden, none_g, none_u = gate_up_swiglu_forward(x, gate, up, False)
+    hidden2, gv, uv = gate_up_swiglu_forward(x, gate, up, True)
+    assert none_g is None and none_u is None and torch.equal(hidden, hidden2)
+    for got, (p, s) in ((gv, gate), (uv, up)):
+        want = x.float() @ dequantize_nf4(p, s).float().t()
+        assert float((got.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+    want = torch.nn.functional.silu(gv.float()) * uv.float()
+    assert float((hidden.float() - want).abs().max()) <= 2e-3 * max(1e-6, float(want.abs().max()))
+    assert cuda_lib.device_status() == 0
+
+
+def test_streaming_forward_many_row_tiles(cuda_lib):
+    """More tiles than two rounds of every SM (the CTAs walk several sets), rows strided and tokens
+    past the last one never written."""
+    from hackaton_b200.nf4 import dequantize_nf4, linear_forward
+
+    n, k = 16 * 16 * 700, 128
+    packed, state = synthetic_weight(n, k, True, seed=3, device="cuda")
+    w = dequantize_nf4(packed, state).float()
+    for m in (1, 3, 20):
+        x = torch.randn(m, k + 8, device="cuda").half()[:, :k]
+        want = x.float() @ w.t()
+        y = linear_forward(x, packed, None, state)
+        assert float((y.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
