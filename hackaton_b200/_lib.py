@@ -18,7 +18,7 @@ EXPORTS = (
     "nf4b200_linear_fwd", "nf4b200_linear_bwd_dx", "nf4b200_lora_down", "nf4b200_lora_grad",
     "nf4b200_workspace_bytes", "nf4b200_linear_fwd_static", "nf4b200_linear_fwd_group",
     "nf4b200_linear_bwd_dx_group", "nf4b200_workspace_bytes_group", "nf4b200_launches_group", "nf4b200_scales16_bytes",
-    "nf4b200_prepare_scales", "nf4b200_lora_down_batch", "nf4b200_lora_grad_batch",
+    "nf4b200_prepare_scales", "nf4b200_lora_down_batch", "nf4b200_lora_grad_batch", "nf4b200_lora_side",
     "nf4b200_set_sm_limit", "nf4b200_gate_up_swiglu_fwd", "nf4b200_gate_up_swiglu_workspace_bytes",
     "nf4b200_swiglu_fwd", "nf4b200_swiglu_bwd", "nf4b200_linear_bwd_dx_swiglu",
     "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", "nf4b200_rmsnorm_fwd", "nf4b200_rmsnorm_bwd",
@@ -44,6 +44,15 @@ class Weight(Structure):
         ("offset", c_void_p), ("code16", c_void_p), ("n_rows", c_int64), ("n_cols", c_int64),
         ("blocksize", c_int32), ("nested_blocksize", c_int32), ("nested", c_int32),
         ("reserved", c_int32), ("scales16", c_void_p),
+    ]
+
+
+class LoraItem(Structure):
+    """nf4b200_lora_item in include/nf4b200.h."""
+    _fields_ = [
+        ("in_", c_void_p), ("c", c_int64), ("ld_in", c_int64), ("p", c_void_p), ("out", c_void_p),
+        ("p16", c_void_p), ("b", c_void_p), ("b16", c_void_p), ("b16t", c_void_p), ("n", c_int64),
+        ("scaling", c_float), ("p_f32", c_int32), ("b_f32", c_int32), ("reserved", c_int32),
     ]
 
 
@@ -99,6 +108,7 @@ def lib() -> ctypes.CDLL:
     pf = POINTER(c_float)
     handle.nf4b200_lora_down_batch.argtypes = [c_int, pv, c_int64, pi64, pi64, pv, pi64, pi64, pf,
                                                pv, c_void_p]
+    handle.nf4b200_lora_side.argtypes = [c_int, POINTER(LoraItem), c_int64, c_void_p, c_size_t, c_void_p]
     handle.nf4b200_lora_grad_batch.argtypes = [c_int, pv, pi64, pi64, pi64, pv, pv, pi64, pi64,
                                                c_void_p]
     handle.nf4b200_set_sm_limit.argtypes = [c_int]

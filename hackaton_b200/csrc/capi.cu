@@ -904,6 +904,45 @@ int nf4b200_lora_down_batch(int count, const void* const* in, int64_t m, const i
     return NF4B200_OK;
 }
 
+int nf4b200_lora_side(int count, const nf4b200_lora_item* items, int64_t m, void* zero,
+                      size_t zero_bytes, void* stream) {
+    DeviceInfo* d = nullptr;
+    int rc = require_sm100(&d);
+    if (rc != NF4B200_OK) return rc;
+    if (count < 1 || count > nf4::LORA_MAX_BATCH)
+        return fail(NF4B200_EINVAL, "lora_side: count %d not in 1..%d", count, nf4::LORA_MAX_BATCH);
+    if (!items || m <= 0) return fail(NF4B200_EINVAL, "lora_side: no items or no rows");
+    if (zero_bytes % 16 != 0 || (zero_bytes && (!zero || !aligned16(zero))))
+        return fail(NF4B200_EINVAL, "lora_side: the region to zero must be 16-byte aligned, in whole 16 bytes");
+    nf4::LoraSide s = {};
+    s.count = count;
+    s.zero = static_cast<uint4*>(zero);
+    s.zero16 = (long long)(zero_bytes / 16);
+    for (int i = 0; i < count; ++i) {
+        const nf4b200_lora_item& it = items[i];
+        if (!it.in || !it.p || !it.out) return fail(NF4B200_EINVAL, "lora_side: NULL pointer in item %d", i);
+        if (it.c <= 0 || it.c % 8 != 0 || it.ld_in < it.c || it.ld_in % 8 != 0 || (it.b && it.n <= 0))
+            return fail(NF4B200_EINVAL, "lora_side: bad shape in item %d (columns and row stride in eights)", i);
+        if (!aligned16(it.in) || !aligned16(it.p) || !aligned16(it.out) || !aligned16(it.p16) ||
+            !aligned16(it.b) || !aligned16(it.b16) || (reinterpret_cast<uintptr_t>(it.b16t) & 1u) != 0)
+            return fail(NF4B200_EINVAL, "lora_side: item %d is not 16-byte aligned", i);
+        nf4::LoraSideItem& q = s.item[i];
+        q.in = static_cast<const __half*>(it.in);
+        q.m = m; q.c = it.c; q.ld_in = it.ld_in;
+        q.p = it.p; q.p_f32 = it.p_f32 != 0;
+        q.scaling = it.scaling;
+        q.out = static_cast<__half*>(it.out);
+        q.p16 = static_cast<__half*>(it.p16);
+        q.b = it.b; q.b_f32 = it.b_f32 != 0; q.n = it.n;
+        q.b16 = static_cast<__half*>(it.b16);
+        q.b16t = static_cast<__half*>(it.b16t);
+    }
+    for (int i = count; i < nf4::LORA_MAX_BATCH; ++i) s.item[i] = s.item[0];
+    cudaError_t e = nf4::launch_lora_side(s, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NF4B200_ECUDA, "lora_side launch: %s", cudaGetErrorString(e));
+    return NF4B200_OK;
+}
+
 int nf4b200_lora_grad_batch(int count, const void* const* z, const int64_t* m, const int64_t* c,
                             const int64_t* ld_z, const void* const* s, float* const* out,
                             const int64_t* o_stride_r, const int64_t* o_stride_c, void* stream) {

@@ -245,6 +245,29 @@ struct LoraDownBatch {
 // One launch when the problems share row count and layout of P; separate launches otherwise.
 cudaError_t launch_lora_down_batch(const LoraDownBatch& b, cudaStream_t stream);
 
+// One direction's side work of a group's adapters (lora.cu, lora_side_kernel): products with the
+// rank-major factor p [16, c], fp16 copies of fp32 factors, the transpose of b, a region to zero.
+struct LoraSideItem {
+    const __half* in;        // [m, c], row pitch ld_in
+    long long m, c, ld_in;
+    const void* p;           // [16, c]
+    __half* out;             // [m, 16]
+    __half* p16;             // fp16 copy of p, or null
+    const void* b;           // [n, 16], or null
+    __half* b16;             // fp16 copy of b, or null
+    __half* b16t;            // its transpose [16, n], or null
+    long long n;
+    float scaling;
+    int p_f32, b_f32;
+};
+struct LoraSide {
+    LoraSideItem item[LORA_MAX_BATCH];
+    int count;
+    uint4* zero;
+    long long zero16;        // 16-byte pieces to zero
+};
+cudaError_t launch_lora_side(const LoraSide& s, cudaStream_t stream);
+
 struct LoraGradArgs {
     const __half* z;
     long long m, c, ld_z;

@@ -35,8 +35,6 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
 constexpr int LD_WARPS = 8;
 constexpr int LD_ROWS = 16;
 constexpr int LD_THREADS = LD_WARPS * 32;
-constexpr int LD_BATCH = 3;   // chunks in flight per warp (16 registers each; two blocks per SM)
-
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                          uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -46,11 +44,37 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <bool RANK_MAJOR>  // P is row-major [16, C] (true) or row-major [C, 16] (false)
+// Eight consecutive values of P as a thread needs them, in P's own type until they are used.
+template <bool F32>
+struct LdP {
+    uint4 q[F32 ? 2 : 1];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < (F32 ? 2 : 1); ++i) q[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __device__ __forceinline__ void load(const void* p, long long idx) {
+        const uint4* s = reinterpret_cast<const uint4*>(static_cast<const char*>(p) + idx * (F32 ? 4 : 2));
+#pragma unroll
+        for (int i = 0; i < (F32 ? 2 : 1); ++i) q[i] = __ldg(s + i);
+    }
+    __device__ __forceinline__ uint4 halves() const {   // fp32 is rounded to nearest
+        if (!F32) return q[0];
+        const uint4 &a = q[0], &b = q[F32 ? 1 : 0];
+        auto two = [](uint32_t x, uint32_t y) {
+            const __half2 h = __floats2half2_rn(__uint_as_float(x), __uint_as_float(y));
+            return *reinterpret_cast<const uint32_t*>(&h);
+        };
+        return make_uint4(two(a.x, a.y), two(a.z, a.w), two(b.x, b.y), two(b.z, b.w));
+    }
+};
+
+// P is row-major [16, C], fp16 or fp32 (RANK_MAJOR), or row-major [C, 16] fp16.
+template <bool RANK_MAJOR, bool F32>
 __device__ __forceinline__ void lora_down_block(const __half* __restrict__ in, long long m,
                                                 long long c, long long ld_in,
-                                                const __half* __restrict__ p, float scaling,
+                                                const void* __restrict__ p, float scaling,
                                                 __half* __restrict__ out) {
+    static_assert(RANK_MAJOR || !F32, "");
     __shared__ float part[LD_WARPS][16][17];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -61,40 +85,47 @@ __device__ __forceinline__ void lora_down_block(const __half* __restrict__ in, l
     const long long chunks = (c + 31) / 32;   // c % 8 == 0 on this path
     const long long ch_begin = chunks * warp / LD_WARPS, ch_end = chunks * (warp + 1) / LD_WARPS;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    // LD_BATCH chunks per round: every load of the round is issued before the first MMA, so a
-    // warp pays one memory round trip per round instead of one per chunk.
-    for (long long ch0 = ch_begin; ch0 < ch_end; ch0 += LD_BATCH) {
-        uint4 a_lo[LD_BATCH], a_hi[LD_BATCH], b_lo[LD_BATCH], b_hi[LD_BATCH];
+    // BATCH chunks are in flight per warp; a chunk's registers take the next request as soon as it has
+    // been used, so the memory latency is paid once and not once per batch.
+    constexpr int BATCH = F32 ? 3 : 4;
+    uint4 a_lo[BATCH], a_hi[BATCH];
+    LdP<F32> b_lo[BATCH], b_hi[BATCH];
+    auto request = [&](int q, long long ch) {
+        const long long col = ch * 32 + t * 8;
+        const bool col_ok = ch < ch_end && col < c;
+        a_lo[q] = a_hi[q] = zero;
+        b_lo[q].zero();
+        b_hi[q].zero();
+        if (!col_ok) return;
+        if (r_lo < m) a_lo[q] = __ldg(reinterpret_cast<const uint4*>(in + r_lo * ld_in + col));
+        if (r_hi < m) a_hi[q] = __ldg(reinterpret_cast<const uint4*>(in + r_hi * ld_in + col));
+        if (RANK_MAJOR) {
+            b_lo[q].load(p, (long long)g * c + col);
+            b_hi[q].load(p, (long long)(g + 8) * c + col);
+        } else {
+            __half lo[8], hi[8];
 #pragma unroll
-        for (int q = 0; q < LD_BATCH; ++q) {
-            const long long col = (ch0 + q) * 32 + t * 8;
-            const bool col_ok = ch0 + q < ch_end && col < c;
-            a_lo[q] = a_hi[q] = b_lo[q] = b_hi[q] = zero;
-            if (col_ok) {
-                if (r_lo < m) a_lo[q] = __ldg(reinterpret_cast<const uint4*>(in + r_lo * ld_in + col));
-                if (r_hi < m) a_hi[q] = __ldg(reinterpret_cast<const uint4*>(in + r_hi * ld_in + col));
-                if (RANK_MAJOR) {
-                    b_lo[q] = __ldg(reinterpret_cast<const uint4*>(p + (long long)g * c + col));
-                    b_hi[q] = __ldg(reinterpret_cast<const uint4*>(p + (long long)(g + 8) * c + col));
-                } else {
-                    __half lo[8], hi[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        lo[e] = __ldg(p + (col + e) * 16 + g);
-                        hi[e] = __ldg(p + (col + e) * 16 + g + 8);
-                    }
-                    b_lo[q] = *reinterpret_cast<const uint4*>(lo);
-                    b_hi[q] = *reinterpret_cast<const uint4*>(hi);
-                }
+            for (int e = 0; e < 8; ++e) {
+                lo[e] = __ldg(static_cast<const __half*>(p) + (col + e) * 16 + g);
+                hi[e] = __ldg(static_cast<const __half*>(p) + (col + e) * 16 + g + 8);
             }
+            b_lo[q].q[0] = *reinterpret_cast<const uint4*>(lo);
+            b_hi[q].q[0] = *reinterpret_cast<const uint4*>(hi);
         }
+    };
 #pragma unroll
-        for (int q = 0; q < LD_BATCH; ++q) {
+    for (int q = 0; q < BATCH; ++q) request(q, ch_begin + q);
+    for (long long ch0 = ch_begin; ch0 < ch_end; ch0 += BATCH) {
+#pragma unroll
+        for (int q = 0; q < BATCH; ++q) {
+            const uint4 al = a_lo[q], ah = a_hi[q], bl = b_lo[q].halves(), bh = b_hi[q].halves();
+            if (ch0 + q + BATCH < ch_end) request(q, ch0 + q + BATCH);
+            else { a_lo[q] = a_hi[q] = zero; b_lo[q].zero(); b_hi[q].zero(); }   // past the end: adds nothing
             // k16 step 0: halves 0,1 | 2,3 ; step 1: halves 4,5 | 6,7
-            mma16816(d0, a_lo[q].x, a_hi[q].x, a_lo[q].y, a_hi[q].y, b_lo[q].x, b_lo[q].y);
-            mma16816(d1, a_lo[q].x, a_hi[q].x, a_lo[q].y, a_hi[q].y, b_hi[q].x, b_hi[q].y);
-            mma16816(d0, a_lo[q].z, a_hi[q].z, a_lo[q].w, a_hi[q].w, b_lo[q].z, b_lo[q].w);
-            mma16816(d1, a_lo[q].z, a_hi[q].z, a_lo[q].w, a_hi[q].w, b_hi[q].z, b_hi[q].w);
+            mma16816(d0, al.x, ah.x, al.y, ah.y, bl.x, bl.y);
+            mma16816(d1, al.x, ah.x, al.y, ah.y, bh.x, bh.y);
+            mma16816(d0, al.z, ah.z, al.w, ah.w, bl.z, bl.w);
+            mma16816(d1, al.z, ah.z, al.w, ah.w, bh.z, bh.w);
         }
     }
     // accumulator layout: d[0],d[1] -> (row g, cols 2t, 2t+1); d[2],d[3] -> (row g+8, same cols)
@@ -121,7 +152,7 @@ lora_down_kernel(const __half* __restrict__ in, long long m, long long c, long l
                  const __half* __restrict__ p, float scaling, __half* __restrict__ out) {
     grid_dep_wait();    // (programmatic dependent launch: the predecessor's results)
     grid_dep_launch();
-    lora_down_block<RANK_MAJOR>(in, m, c, ld_in, p, scaling, out);
+    lora_down_block<RANK_MAJOR, false>(in, m, c, ld_in, p, scaling, out);
 }
 
 // Several lora_down problems with the same row count in one launch: blockIdx.y picks the problem.
@@ -131,7 +162,76 @@ lora_down_batch_kernel(const __grid_constant__ LoraDownBatch b) {
     grid_dep_wait();
     grid_dep_launch();
     const LoraDownArgs& a = b.item[blockIdx.y];
-    lora_down_block<RANK_MAJOR>(a.in, a.m, a.c, a.ld_in, a.p, a.scaling, a.out);
+    lora_down_block<RANK_MAJOR, false>(a.in, a.m, a.c, a.ld_in, a.p, a.scaling, a.out);
+}
+
+// What one direction of a group's adapters needs before its GEMM, in one launch: the products of
+// lora_down (P fp32 or fp16, rank-major; blockIdx.y picks the problem) and, in the last slice of the
+// grid, fp16 copies of fp32 factors, the transpose of B that the gradient's product reads with 16-byte
+// loads, and zeros for the gradients that are summed atomically later. Each of these was a launch of its
+// own (eight casts and a fill per group, 1.4 to 2 us each on the GPU and several on the host; the
+// strided reads of B [C, 16] made the backward product 6.4 us at 2048 x 1536, now 4.5).
+template <bool F32>
+__device__ __forceinline__ void lora_factor_b(const void* b, long long row, __half (&h)[16]) {
+    LdP<F32> lo, hi;
+    lo.load(b, row * 16);
+    hi.load(b, row * 16 + 8);
+    const uint4 v[2] = {lo.halves(), hi.halves()};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = reinterpret_cast<const __half*>(v)[i];
+}
+
+__global__ void __launch_bounds__(LD_THREADS)
+lora_side_kernel(const __grid_constant__ LoraSide s) {
+    grid_dep_wait();
+    grid_dep_launch();
+    if ((int)blockIdx.y < s.count) {
+        const LoraSideItem& a = s.item[blockIdx.y];
+        if ((long long)blockIdx.x * LD_ROWS >= a.m) return;
+        if (a.p_f32) lora_down_block<true, true>(a.in, a.m, a.c, a.ld_in, a.p, a.scaling, a.out);
+        else         lora_down_block<true, false>(a.in, a.m, a.c, a.ld_in, a.p, a.scaling, a.out);
+        return;
+    }
+    const long long tid = (long long)blockIdx.x * LD_THREADS + threadIdx.x;
+    const long long stride = (long long)gridDim.x * LD_THREADS;
+    for (long long i = tid; i < s.zero16; i += stride) s.zero[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < s.count; ++k) {
+        const LoraSideItem& a = s.item[k];
+        if (a.p16 != nullptr && a.p_f32) {
+            for (long long i = tid; i < 2 * a.c; i += stride) {   // 16 * c values, 8 at a time
+                LdP<true> v;
+                v.load(a.p, i * 8);
+                reinterpret_cast<uint4*>(a.p16)[i] = v.halves();
+            }
+        }
+        if (a.b == nullptr) continue;
+        for (long long r = tid; r < a.n; r += stride) {
+            __align__(16) __half h[16];
+            if (a.b_f32) lora_factor_b<true>(a.b, r, h);
+            else         lora_factor_b<false>(a.b, r, h);
+            if (a.b16 != nullptr) {
+                reinterpret_cast<uint4*>(a.b16)[r * 2] = reinterpret_cast<const uint4*>(h)[0];
+                reinterpret_cast<uint4*>(a.b16)[r * 2 + 1] = reinterpret_cast<const uint4*>(h)[1];
+            }
+            if (a.b16t != nullptr)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) a.b16t[j * a.n + r] = h[j];
+        }
+    }
+}
+
+cudaError_t launch_lora_side(const LoraSide& s, cudaStream_t stream) {
+    bool extra = s.zero16 > 0;
+    long long blocks = 0;
+    for (int i = 0; i < s.count; ++i) {
+        const LoraSideItem& a = s.item[i];
+        extra = extra || a.p16 != nullptr || a.b != nullptr;
+        const long long need = (a.m + LD_ROWS - 1) / LD_ROWS;
+        blocks = need > blocks ? need : blocks;
+    }
+    if (extra && blocks < 32) blocks = 32;   // few rows: the copies still spread over some SMs
+    return launch_pdl(lora_side_kernel, dim3((unsigned)blocks, (unsigned)(s.count + (extra ? 1 : 0))),
+                      dim3(LD_THREADS), 0, stream, s);
 }
 
 // Layout-agnostic variant (any strides, any alignment): one thread per output element.

@@ -20,7 +20,7 @@ from typing import Optional, Sequence
 import torch
 
 from . import _lib
-from .lora import RANK, lora_down_batch, lora_grad_batch
+from .lora import RANK, grad_buffer, lora_grad_batch, lora_side
 from .nf4 import _require, _rows_view, _stream_ptr, _ws_buffers, weight_ref
 
 MAX_GROUP = 4
@@ -142,21 +142,23 @@ class NF4LinearGroup(torch.autograd.Function):
         biases, las, lbs = params[0::3], params[1::3], params[2::3]
         xas, b16 = [None] * n, [None] * n
         with_lora = [i for i, a in enumerate(las) if a is not None]
-        if with_lora:  # every adapter's scaling * x . Aᵀ in one launch
-            downs = lora_down_batch([x] * len(with_lora), [las[i] for i in with_lora], True,
-                                    [projs[i].scaling for i in with_lora])
-            for i, xa in zip(with_lora, downs):
-                xas[i] = xa
-                b16[i] = lbs[i].detach().to(torch.float16).contiguous()
+        kept = {}
+        if with_lora:  # every adapter's scaling * x . Aᵀ and the fp16 factors in one launch
+            train = any(ctx.needs_input_grad)
+            downs, a16s, b16s, b16ts = lora_side(
+                [x] * len(with_lora), [las[i] for i in with_lora], [projs[i].scaling for i in with_lora],
+                [lbs[i] for i in with_lora], transpose=train)
+            for i, xa, a, b, bt in zip(with_lora, downs, a16s, b16s, b16ts):
+                xas[i], b16[i], kept[i] = xa, b, (a, bt)
         ys = linear_forward_group(x, [(pr.packed, pr.state) for pr in projs], biases, xas, b16)
         ctx.projs, ctx.n = projs, n
         ctx.bias_dtypes = [None if b is None else b.dtype for b in biases]
         ctx.has_lora = [a is not None for a in las]
-        saved = [x]
-        for a, b, xa in zip(las, lbs, xas):
-            if a is not None:
-                saved += [a, b, xa]
-        ctx.save_for_backward(*saved)
+        if any(ctx.needs_input_grad):
+            saved = [x]
+            for i in with_lora:
+                saved += [las[i], lbs[i], xas[i], *kept[i]]
+            ctx.save_for_backward(*saved)
         return tuple(ys)
 
     @staticmethod
@@ -166,33 +168,35 @@ class NF4LinearGroup(torch.autograd.Function):
         projs = ctx.projs
         lora = []
         for has in ctx.has_lora:
-            lora.append((saved.pop(0), saved.pop(0), saved.pop(0)) if has else None)
+            lora.append(tuple(saved.pop(0) for _ in range(5)) if has else None)   # A, B, xa, A16, Bᵀ16
         grads = [g if g is not None else
                  torch.zeros(*x.shape[:-1], pr.state.shape[0], dtype=torch.float16, device=x.device)
                  for g, pr in zip(grads, projs)]
         us, a16 = [None] * len(projs), [None] * len(projs)
         with_lora = [i for i, lo in enumerate(lora) if lo is not None]
+        # all LoRA weight gradients of the group in one launch, summed into a zeroed buffer
+        jobs = []  # (z, s or None for u, rank-major output, projection, "a" | "b")
+        for i in with_lora:
+            if ctx.needs_input_grad[3 + 3 * i]:
+                jobs.append((x, None, True, i, "a"))
+            if ctx.needs_input_grad[4 + 3 * i]:
+                jobs.append((grads[i], lora[i][2], False, i, "b"))
+        flat = grad_buffer(jobs, x.device) if jobs else None
         if with_lora:  # every adapter's scaling * dy . B in one launch
-            downs = lora_down_batch([grads[i] for i in with_lora], [lora[i][1] for i in with_lora],
-                                    False, [projs[i].scaling for i in with_lora])
+            downs, *_ = lora_side([grads[i] for i in with_lora], [lora[i][4] for i in with_lora],
+                                  [projs[i].scaling for i in with_lora], zero=flat)
             for i, u in zip(with_lora, downs):
                 us[i] = u
-                a16[i] = lora[i][0].detach().to(torch.float16).contiguous()
+                a16[i] = lora[i][3]
         grad_x = None
         if ctx.needs_input_grad[0]:
             grad_x = linear_backward_dx_group(grads, [(pr.packed, pr.state) for pr in projs], us, a16)
-        # all LoRA weight gradients of the group in one launch
-        jobs = []  # (projection, "a" | "b", z, s, rank-major output)
-        for i in with_lora:
-            if ctx.needs_input_grad[3 + 3 * i]:
-                jobs.append((i, "a", x, us[i], True))
-            if ctx.needs_input_grad[4 + 3 * i]:
-                jobs.append((i, "b", grads[i], lora[i][2], False))
         wgrads = {}
         if jobs:
-            res = lora_grad_batch([j[2] for j in jobs], [j[3] for j in jobs], [j[4] for j in jobs])
+            res = lora_grad_batch([j[0] for j in jobs], [us[j[3]] if j[1] is None else j[1] for j in jobs],
+                                  [j[2] for j in jobs], flat)
             for j, r in zip(jobs, res):
-                wgrads[(j[0], j[1])] = r
+                wgrads[j[3:]] = r
         out = [grad_x, None]
         for i, (g, pr, lo) in enumerate(zip(grads, projs, lora)):
             gb = ga = gbb = None

@@ -94,17 +94,92 @@ def lora_down_batch(inputs, ps, p_is_rank_major, scalings):
     return outs
 
 
-def lora_grad_batch(zs, ss, rank_major_outs):
+def _factor(p):
+    """A LoRA factor as the side kernel reads it: contiguous, 16-byte aligned fp32 or fp16."""
+    p = p.detach()
+    if p.dtype not in (torch.float32, torch.float16):
+        p = p.to(torch.float16)
+    p = p.contiguous()
+    return p if p.data_ptr() % 16 == 0 else p.clone()
+
+
+def lora_side(inputs, ps, scalings, bs=None, transpose=False, zero=None):
+    """One launch (nf4b200_lora_side) for what a direction of several adapters needs besides the
+    GEMM: scaling * input . pᵀ for rank-major factors p [16, C] (fp32 or fp16; the inputs share their
+    row count) and fp16 copies of p. With `bs` ([N, 16] each) also their fp16 copies and, with
+    `transpose`, fp16 [16, N] transposes. `zero`: an fp32 buffer (a multiple of 4 elements) to fill with zeros.
+    Returns (products, p16s, b16s, b16ts)."""
+    n = len(inputs)
+    items = (_lib.LoraItem * n)()
+    keep, p16s, b16s, b16ts = [], [], [], []
+    device = inputs[0].device
+    half = dict(dtype=torch.float16, device=device)
+    m = None
+    for i, (inp, p, scaling) in enumerate(zip(inputs, ps, scalings)):
+        c = inp.shape[-1]
+        i2, p = _rows_view(inp, c), _factor(p)
+        assert tuple(p.shape) == (RANK, c), (p.shape, c)
+        if m is None:
+            m = i2.shape[0]
+            products = torch.empty((n, m, RANK), **half)
+        assert i2.shape[0] == m
+        it = items[i]
+        it.in_, it.c, it.ld_in, it.p, it.scaling = i2.data_ptr(), c, i2.stride(0), p.data_ptr(), float(scaling)
+        it.out = products.data_ptr() + i * m * RANK * 2
+        it.p_f32 = p.dtype == torch.float32
+        p16 = torch.empty((RANK, c), **half) if it.p_f32 else p
+        it.p16 = p16.data_ptr() if it.p_f32 else None
+        p16s.append(p16)
+        keep += [i2, p]
+        if bs is not None:
+            b = _factor(bs[i])
+            rows = b.shape[0]
+            assert tuple(b.shape) == (rows, RANK), b.shape
+            it.b, it.n, it.b_f32 = b.data_ptr(), rows, b.dtype == torch.float32
+            b16 = torch.empty((rows, RANK), **half) if it.b_f32 else b
+            it.b16 = b16.data_ptr() if it.b_f32 else None
+            b16t = torch.empty((RANK, rows), **half) if transpose else None
+            it.b16t = None if b16t is None else b16t.data_ptr()
+            b16s.append(b16)
+            b16ts.append(b16t)
+            keep.append(b)
+    if m == 0:   # nothing to multiply: the copies and zeros by torch
+        for i, p in enumerate(ps):
+            p16s[i].copy_(p.detach())
+            if bs is not None:
+                b16s[i].copy_(bs[i].detach())
+                if transpose:
+                    b16ts[i].copy_(bs[i].detach().t())
+        if zero is not None:
+            zero.zero_()
+    else:
+        with torch.cuda.device(device):
+            _lib.check(_lib.lib().nf4b200_lora_side(
+                n, items, m, None if zero is None else zero.data_ptr(),
+                0 if zero is None else zero.numel() * 4, _stream_ptr(device)))
+    return list(products.unbind(0)), p16s, b16s, b16ts
+
+
+def grad_buffer(jobs, device):
+    """Uninitialised fp32 buffer for the results of `lora_grad_batch` over jobs (z, s, rank-major):
+    256-byte aligned pieces, to be zeroed before."""
+    return torch.empty(sum((z.shape[-1] * RANK + 63) // 64 * 64 for z, *_ in jobs), dtype=torch.float32,
+                       device=device)
+
+
+def lora_grad_batch(zs, ss, rank_major_outs, flat=None):
     """lora_grad for several (z, s) pairs in one launch (nf4b200_lora_grad_batch); one zeroed
-    fp32 buffer holds all results. Returns the list of gradients, [16, C] or [C, 16] each."""
+    fp32 buffer (`flat`, from `grad_buffer`, or a new one) holds all results. Returns the list of
+    gradients, [16, C] or [C, 16] each."""
     n = len(zs)
-    if n == 1:
+    if n == 1 and flat is None:
         return [lora_grad(zs[0], ss[0], rank_major_outs[0])]
     z2s = [_rows_view(z, z.shape[-1]) for z in zs]
     cs = [z.shape[-1] for z in zs]
     device = zs[0].device
     sizes = [(c * RANK + 63) // 64 * 64 for c in cs]         # 256-byte aligned pieces
-    flat = torch.zeros(sum(sizes), dtype=torch.float32, device=device)
+    if flat is None:
+        flat = torch.zeros(sum(sizes), dtype=torch.float32, device=device)
     outs, at = [], 0
     for c, size, rm in zip(cs, sizes, rank_major_outs):
         outs.append(flat[at:at + c * RANK].view((RANK, c) if rm else (c, RANK)))
@@ -128,24 +203,33 @@ class NF4LoRALinear(torch.autograd.Function):
     def forward(ctx, x, x_lora, packed, bias, state, lora_a, lora_b, scaling):
         same = x_lora is x or (x_lora.data_ptr() == x.data_ptr() and x_lora.shape == x.shape
                                and x_lora.stride() == x.stride())
-        xa = lora_down(x_lora, lora_a, True, scaling)          # scaling * x_l . Aᵀ  [M,16]
-        b16 = lora_b.detach().to(torch.float16).contiguous()
+        # scaling * x_l . Aᵀ [M, 16], fp16 A and B, and Bᵀ for the gradient's product
+        (xa,), (a16,), (b16,), (b16t,) = lora_side([x_lora], [lora_a], [scaling], [lora_b],
+                                                   transpose=any(ctx.needs_input_grad))
         y = linear_forward(x, packed, bias, state, xa=xa, lora_b=b16)
         ctx.packed, ctx.state, ctx.scaling, ctx.same = packed, state, float(scaling), same
         ctx.bias_dtype = None if bias is None else bias.dtype
-        ctx.save_for_backward(x_lora, xa, lora_a, lora_b)
+        if b16t is not None:
+            ctx.save_for_backward(x_lora, xa, lora_a, lora_b, a16, b16t)
         return y
 
     @staticmethod
     def backward(ctx, grad_output):
-        x_lora, xa, lora_a, lora_b = ctx.saved_tensors
+        x_lora, xa, lora_a, lora_b, a16, b16t = ctx.saved_tensors
         need_x, need_xl = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         need_a, need_b = ctx.needs_input_grad[5], ctx.needs_input_grad[6]
         grad_x = grad_xl = grad_bias = grad_a = grad_b = None
         u = None
-        if need_x or need_xl or need_a:
-            u = lora_down(grad_output, lora_b, False, ctx.scaling)   # scaling * dy . B  [M,16]
-        a16 = lora_a.detach().to(torch.float16).contiguous()
+        jobs = []   # (z, s, rank-major output): the two factors' gradients in one launch
+        if need_a:
+            jobs.append((x_lora, None, True))
+        if need_b:
+            jobs.append((grad_output, xa, False))
+        flat = grad_buffer(jobs, grad_output.device) if jobs else None
+        if need_x or need_xl or need_a:      # scaling * dy . B [M, 16]
+            (u,), *_ = lora_side([grad_output], [b16t], [ctx.scaling], zero=flat)
+        elif flat is not None:
+            flat.zero_()
         if ctx.same:
             if need_x or need_xl:
                 grad_x = linear_backward_dx(grad_output, ctx.packed, ctx.state, u=u, lora_a=a16)
@@ -154,10 +238,13 @@ class NF4LoRALinear(torch.autograd.Function):
                 grad_x = linear_backward_dx(grad_output, ctx.packed, ctx.state)
             if need_xl:  # the dropout branch keeps its own gradient: u . A
                 grad_xl = (u.reshape(-1, RANK) @ a16).reshape(x_lora.shape)
-        if need_a:
-            grad_a = lora_grad(x_lora, u, True).to(lora_a.dtype)
-        if need_b:
-            grad_b = lora_grad(grad_output, xa, False).to(lora_b.dtype)
+        if jobs:
+            res = lora_grad_batch([j[0] for j in jobs], [u if j[1] is None else j[1] for j in jobs],
+                                  [j[2] for j in jobs], flat)
+            if need_a:
+                grad_a = res[0].to(lora_a.dtype)
+            if need_b:
+                grad_b = res[-1].to(lora_b.dtype)
         if ctx.needs_input_grad[3]:
             grad_bias = grad_output.reshape(-1, grad_output.shape[-1]).sum(0, dtype=ctx.bias_dtype)
         return grad_x, grad_xl, None, grad_bias, None, grad_a, grad_b, None

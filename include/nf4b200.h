@@ -362,6 +362,32 @@ int nf4b200_lora_grad_batch(int count, const void* const* z, const int64_t* m, c
                             const int64_t* ld_z, const void* const* s, float* const* out,
                             const int64_t* o_stride_r, const int64_t* o_stride_c, void* stream);
 
+/*
+ * Everything one direction of a group's adapters needs besides the GEMM, in one launch: per item
+ *   out[m, 16] = scaling * in[m, c] . p^T        p row-major [16, c], fp32 (p_f32) or fp16
+ *   p16  [16, c]  fp16 copy of p                 (NULL: not wanted; only made from an fp32 p)
+ *   b16  [n, 16]  fp16 copy of b, and its transpose b16t [16, n]   (NULL: not wanted)
+ * and `zero_bytes` bytes of zeros at `zero` (the fp32 gradients nf4b200_lora_grad_batch adds to).
+ * fp32 values are rounded to nearest. in, p, out, p16, b, b16 and zero must be 16-byte aligned,
+ * c and ld_in multiples of 8, zero_bytes a multiple of 16.
+ */
+typedef struct nf4b200_lora_item {
+    const void* in;
+    int64_t c, ld_in;
+    const void* p;
+    void* out;
+    void* p16;
+    const void* b;
+    void* b16;
+    void* b16t;
+    int64_t n;
+    float scaling;
+    int32_t p_f32, b_f32, reserved;
+} nf4b200_lora_item;
+int nf4b200_lora_side(int count, const nf4b200_lora_item* items, int64_t m, void* zero,
+                      size_t zero_bytes, void* stream);
+
+
 #ifdef __cplusplus
 }
 #endif

@@ -103,3 +103,41 @@ def test_batched_lora_kernels_match_single(cuda_lib):
         assert g.shape == w.shape
         # fp32 atomics: the order of the block sums is not fixed
         assert (g - w).abs().max() <= 1e-4 * w.abs().max().clamp_min(1.0)
+
+
+@pytest.mark.parametrize("m", [1, 15, 16, 17, 300])
+@pytest.mark.parametrize("c,n", [(8, 8), (64, 264), (1544, 1536), (3584, 512)])   # ragged chunks of 32 columns
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_side_kernel(cuda_lib, m, c, n, dtype):
+    """Products, fp16 copies, transpose and zeros of nf4b200_lora_side: copies exactly torch's rounding;
+    products against 64-bit sums of the fp16 factors (fp32 accumulation and one fp16 rounding)."""
+    from hackaton_b200.lora import lora_side
+
+    g = torch.Generator(device="cuda").manual_seed(m + c)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    xs = [rand(m, c).half(), rand(m, c + 8).half()[:, :c]]
+    ps, bs = [rand(16, c).to(dtype) for _ in range(2)], [rand(n, 16).to(dtype) for _ in range(2)]
+    zero = rand(52)
+    outs, p16s, b16s, b16ts = lora_side(xs, ps, [2.0, 0.5], bs, transpose=True, zero=zero)
+    for x, p, b, s, o, p16, b16, bt in zip(xs, ps, bs, (2.0, 0.5), outs, p16s, b16s, b16ts):
+        assert torch.equal(p16, p.half()) and torch.equal(b16, b.half()) and torch.equal(bt, b.half().t())
+        want = s * x.double() @ p.half().double().t()
+        scale = s * (x.double().abs() @ p.half().double().abs().t())
+        assert ((o.double() - want).abs() <= 2.0 ** -11 * want.abs() + 1e-6 * scale + 1e-7).all()
+    assert not zero.any()
+
+
+def test_unmodified_when_only_b_needs_a_gradient(cuda_lib):
+    """The gradient buffer is zeroed on every path (here: no product in the backward zeroes it)."""
+    from hackaton_b200 import nf4_lora_linear
+
+    packed, state = synthetic_weight(64, 128, True, seed=1, device="cuda")
+    x = torch.randn(40, 128, device="cuda").half()
+    a, b = torch.randn(16, 128, device="cuda"), torch.randn(64, 16, device="cuda", requires_grad=True)
+    junk = torch.full((1 << 16,), 7.0, device="cuda")
+    del junk                                   # a later allocation of this size is not zero
+    y = nf4_lora_linear(x, packed, None, state, a, b, 2.0)
+    gy = torch.randn_like(y)
+    grad, = torch.autograd.grad(y, b, gy)
+    want = gy.double().t() @ (2.0 * x.double() @ a.half().double().t()).half().double()
+    assert float((grad.double() - want).abs().max()) <= 1e-3 * float(want.abs().max())
