@@ -152,6 +152,24 @@ def lib() -> ctypes.CDLL:
     return handle
 
 
+_host_module = None
+
+
+def host():
+    """The extension module that makes the frequent calls with torch tensors (csrc/host.cpp)."""
+    global _host_module
+    if _host_module is None:
+        lib()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise RuntimeError(
+                "hackaton_b200/_host.so is missing or does not fit the installed torch: build it with "
+                "`python -m hackaton_b200.build` (needs nvcc and g++)") from e
+        _host_module = _host
+    return _host_module
+
+
 def check(status: int) -> None:
     if status != 0:
         raise Nf4Error(status, lib().nf4b200_last_error().decode("utf-8", "replace"))

@@ -1,4 +1,5 @@
-"""Builds libnf4b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libnf4b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and _host.so (the
+Python module csrc/host.cpp, which calls it with torch tensors) with g++.
 
     python -m hackaton_b200.build            # build if sources are newer than the library
     python -m hackaton_b200.build --force
@@ -12,11 +13,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libnf4b200.so"
+HOST = PKG / "_host.so"
 SOURCES = ["capi.cu", "cross_entropy.cu", "dequant.cu", "gemm.cu", "gemv.cu", "lora.cu", "rmsnorm.cu", "rope.cu", "selftest.cu", "static_scratch.cu", "swiglu.cu"]
 
 NVCC_FLAGS = [
@@ -42,8 +45,30 @@ def _stale() -> bool:
     return any(p.stat().st_mtime > built for p in deps)
 
 
+def build_host(force: bool = False) -> Path:
+    """The extension module, against the headers and libraries of the torch that is installed."""
+    src, header = CSRC / "host.cpp", PKG.parent / "include" / "nf4b200.h"
+    if not force and HOST.exists() and HOST.stat().st_mtime >= max(src.stat().st_mtime, header.stat().st_mtime):
+        return HOST
+    import torch
+
+    base = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    tmp = HOST.with_suffix(".so.tmp")
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", str(src), "-o", str(tmp),
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-I{base}/include", f"-I{base}/include/torch/csrc/api/include",
+           f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
+           f"-L{base}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+           f"-L{PKG}", "-l:libnf4b200.so", "-Wl,-rpath,$ORIGIN"]
+    subprocess.run(cmd, check=True)
+    os.replace(tmp, HOST)
+    return HOST
+
+
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     if not force and not _stale():
+        build_host()
         return LIB
     flags = [f for f in NVCC_FLAGS if f != "--use_fast_math=false"]
     flags += os.environ.get("NF4B200_NVCC_FLAGS", "").split()   # e.g. -DNF4B200_TRACE for tuning
@@ -71,6 +96,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     link = [_nvcc(), "-shared", "-o", str(tmp), *objs, "-lcudart"]
     subprocess.run(link, check=True)
     os.replace(tmp, LIB)
+    build_host(force)
     return LIB
 
 

@@ -21,7 +21,7 @@ import torch
 
 from . import _lib
 from .lora import RANK, grad_buffer, lora_grad_batch, lora_side
-from .nf4 import _require, _rows_view, _stream_ptr, _ws_buffers, weight_ref
+from .nf4 import _require, _rows, _scratch, weight_ref
 
 MAX_GROUP = 4
 
@@ -41,6 +41,8 @@ _ws_need = {}
 
 
 def _workspace(device, rows, cols, m, backward):
+    if m == 0:
+        return None, 0
     key = (device.index, tuple(rows), cols, m, backward)
     need = _ws_need.get(key)
     if need is None:
@@ -52,12 +54,7 @@ def _workspace(device, rows, cols, m, backward):
         _ws_need[key] = need
     if need == 0:
         return None, 0
-    skey = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _ws_buffers.get(skey)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
-        _ws_buffers[skey] = buf
-    return buf.data_ptr(), buf.numel()
+    return _scratch(device, need)
 
 
 def _refs(items):
@@ -74,62 +71,33 @@ def _refs(items):
     return refs
 
 
-def _ptr_array(values):
-    return (ctypes.c_void_p * len(values))(*[None if v is None else v.data_ptr() for v in values])
-
-
 def linear_forward_group(x, weights: Sequence, biases=None, xas=None, lora_bs=None):
     """weights: [(packed, state), ...]. Returns the list of outputs y_i = x . W_iᵀ (+ ...)."""
     refs = _refs(weights)
-    n = len(refs)
+    none = [None] * len(refs)
     if x.dtype != torch.float16:
         raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {x.dtype}")
     cols = refs[0].cols
-    x2 = _rows_view(x, cols)
-    m = x2.shape[0]
-    ys = [torch.empty((m, r.rows), dtype=torch.float16, device=x.device) for r in refs]
-    if m == 0:
-        return [y.reshape(*x.shape[:-1], y.shape[1]) for y in ys]
-    biases = [None] * n if biases is None else [None if b is None else b.to(torch.float16).contiguous()
-                                                 for b in biases]
-    xas = [None] * n if xas is None else list(xas)
-    lora_bs = [None] * n if lora_bs is None else list(lora_bs)
-    ws, ws_bytes = _workspace(x.device, [r.rows for r in refs], cols, m, False)
-    w_arr = (ctypes.POINTER(_lib.Weight) * n)(*[ctypes.pointer(r.struct) for r in refs])
-    ldy = (ctypes.c_int64 * n)(*[y.stride(0) for y in ys])
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().nf4b200_linear_fwd_group(
-            n, w_arr, x2.data_ptr(), m, x2.stride(0), _ptr_array(biases), _ptr_array(xas),
-            _ptr_array(lora_bs), _ptr_array(ys), ldy, ws, ws_bytes, _stream_ptr(x.device)))
-    return [y.reshape(*x.shape[:-1], y.shape[1]) for y in ys]
+    if x.shape[-1] != cols:
+        raise ValueError(f"input has {x.shape[-1]} features, weights expect {cols}")
+    ws, ws_bytes = _workspace(x.device, [r.rows for r in refs], cols, _rows(x), False)
+    return _lib.host().linear_fwd_group(
+        [r.address for r in refs], x, none if biases is None else list(biases), none if xas is None else list(xas),
+        none if lora_bs is None else list(lora_bs), ws or 0, ws_bytes)
 
 
 def linear_backward_dx_group(grads: Sequence[torch.Tensor], weights: Sequence, us=None, lora_as=None):
     """dx = Σ_i grads[i] . W_i (+ u_i . lora_a_i). grads[i]: fp16 [..., N_i]."""
     refs = _refs(weights)
-    n = len(refs)
-    g2 = []
+    none = [None] * len(refs)
     for g, r in zip(grads, refs):
         if g.dtype != torch.float16:
             raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {g.dtype}")
-        g2.append(_rows_view(g, r.rows))
-    m = g2[0].shape[0]
-    cols = refs[0].cols
-    dx = torch.empty((m, cols), dtype=torch.float16, device=g2[0].device)
-    lead = grads[0].shape[:-1]
-    if m == 0:
-        return dx.reshape(*lead, cols)
-    us = [None] * n if us is None else list(us)
-    lora_as = [None] * n if lora_as is None else list(lora_as)
-    device = g2[0].device
-    ws, ws_bytes = _workspace(device, [r.rows for r in refs], cols, m, True)
-    w_arr = (ctypes.POINTER(_lib.Weight) * n)(*[ctypes.pointer(r.struct) for r in refs])
-    ldg = (ctypes.c_int64 * n)(*[g.stride(0) for g in g2])
-    with torch.cuda.device(device):
-        _lib.check(_lib.lib().nf4b200_linear_bwd_dx_group(
-            n, w_arr, _ptr_array(g2), m, ldg, _ptr_array(us), _ptr_array(lora_as), dx.data_ptr(),
-            dx.stride(0), ws, ws_bytes, _stream_ptr(device)))
-    return dx.reshape(*lead, cols)
+        if g.shape[-1] != r.rows:
+            raise ValueError(f"gradient has {g.shape[-1]} features, weight gives {r.rows}")
+    ws, ws_bytes = _workspace(grads[0].device, [r.rows for r in refs], refs[0].cols, _rows(grads[0]), True)
+    return _lib.host().linear_bwd_dx_group([r.address for r in refs], list(grads), none if us is None else list(us),
+                                           none if lora_as is None else list(lora_as), ws or 0, ws_bytes)
 
 
 class NF4LinearGroup(torch.autograd.Function):

@@ -94,70 +94,13 @@ def lora_down_batch(inputs, ps, p_is_rank_major, scalings):
     return outs
 
 
-def _factor(p):
-    """A LoRA factor as the side kernel reads it: contiguous, 16-byte aligned fp32 or fp16."""
-    p = p.detach()
-    if p.dtype not in (torch.float32, torch.float16):
-        p = p.to(torch.float16)
-    p = p.contiguous()
-    return p if p.data_ptr() % 16 == 0 else p.clone()
-
-
 def lora_side(inputs, ps, scalings, bs=None, transpose=False, zero=None):
     """One launch (nf4b200_lora_side) for what a direction of several adapters needs besides the
     GEMM: scaling * input . pᵀ for rank-major factors p [16, C] (fp32 or fp16; the inputs share their
     row count) and fp16 copies of p. With `bs` ([N, 16] each) also their fp16 copies and, with
     `transpose`, fp16 [16, N] transposes. `zero`: an fp32 buffer (a multiple of 4 elements) to fill with zeros.
     Returns (products, p16s, b16s, b16ts)."""
-    n = len(inputs)
-    items = (_lib.LoraItem * n)()
-    keep, p16s, b16s, b16ts = [], [], [], []
-    device = inputs[0].device
-    half = dict(dtype=torch.float16, device=device)
-    m = None
-    for i, (inp, p, scaling) in enumerate(zip(inputs, ps, scalings)):
-        c = inp.shape[-1]
-        i2, p = _rows_view(inp, c), _factor(p)
-        assert tuple(p.shape) == (RANK, c), (p.shape, c)
-        if m is None:
-            m = i2.shape[0]
-            products = torch.empty((n, m, RANK), **half)
-        assert i2.shape[0] == m
-        it = items[i]
-        it.in_, it.c, it.ld_in, it.p, it.scaling = i2.data_ptr(), c, i2.stride(0), p.data_ptr(), float(scaling)
-        it.out = products.data_ptr() + i * m * RANK * 2
-        it.p_f32 = p.dtype == torch.float32
-        p16 = torch.empty((RANK, c), **half) if it.p_f32 else p
-        it.p16 = p16.data_ptr() if it.p_f32 else None
-        p16s.append(p16)
-        keep += [i2, p]
-        if bs is not None:
-            b = _factor(bs[i])
-            rows = b.shape[0]
-            assert tuple(b.shape) == (rows, RANK), b.shape
-            it.b, it.n, it.b_f32 = b.data_ptr(), rows, b.dtype == torch.float32
-            b16 = torch.empty((rows, RANK), **half) if it.b_f32 else b
-            it.b16 = b16.data_ptr() if it.b_f32 else None
-            b16t = torch.empty((RANK, rows), **half) if transpose else None
-            it.b16t = None if b16t is None else b16t.data_ptr()
-            b16s.append(b16)
-            b16ts.append(b16t)
-            keep.append(b)
-    if m == 0:   # nothing to multiply: the copies and zeros by torch
-        for i, p in enumerate(ps):
-            p16s[i].copy_(p.detach())
-            if bs is not None:
-                b16s[i].copy_(bs[i].detach())
-                if transpose:
-                    b16ts[i].copy_(bs[i].detach().t())
-        if zero is not None:
-            zero.zero_()
-    else:
-        with torch.cuda.device(device):
-            _lib.check(_lib.lib().nf4b200_lora_side(
-                n, items, m, None if zero is None else zero.data_ptr(),
-                0 if zero is None else zero.numel() * 4, _stream_ptr(device)))
-    return list(products.unbind(0)), p16s, b16s, b16ts
+    return _lib.host().lora_side(inputs, ps, scalings, [] if bs is None else bs, transpose, zero)
 
 
 def grad_buffer(jobs, device):
@@ -171,28 +114,11 @@ def lora_grad_batch(zs, ss, rank_major_outs, flat=None):
     """lora_grad for several (z, s) pairs in one launch (nf4b200_lora_grad_batch); one zeroed
     fp32 buffer (`flat`, from `grad_buffer`, or a new one) holds all results. Returns the list of
     gradients, [16, C] or [C, 16] each."""
-    n = len(zs)
-    if n == 1 and flat is None:
+    if len(zs) == 1 and flat is None:
         return [lora_grad(zs[0], ss[0], rank_major_outs[0])]
-    z2s = [_rows_view(z, z.shape[-1]) for z in zs]
-    cs = [z.shape[-1] for z in zs]
-    device = zs[0].device
-    sizes = [(c * RANK + 63) // 64 * 64 for c in cs]         # 256-byte aligned pieces
     if flat is None:
-        flat = torch.zeros(sum(sizes), dtype=torch.float32, device=device)
-    outs, at = [], 0
-    for c, size, rm in zip(cs, sizes, rank_major_outs):
-        outs.append(flat[at:at + c * RANK].view((RANK, c) if rm else (c, RANK)))
-        at += size
-    vp, i64 = ctypes.c_void_p, ctypes.c_int64
-    with torch.cuda.device(device):
-        _lib.check(_lib.lib().nf4b200_lora_grad_batch(
-            n, _arr(vp, [t.data_ptr() for t in z2s]), _arr(i64, [t.shape[0] for t in z2s]),
-            _arr(i64, cs), _arr(i64, [t.stride(0) for t in z2s]),
-            _arr(vp, [t.data_ptr() for t in ss]), _arr(vp, [t.data_ptr() for t in outs]),
-            _arr(i64, [c if rm else 1 for c, rm in zip(cs, rank_major_outs)]),
-            _arr(i64, [1 if rm else RANK for rm in rank_major_outs]), _stream_ptr(device)))
-    return outs
+        flat = grad_buffer([(z,) for z in zs], zs[0].device).zero_()
+    return _lib.host().lora_grad_batch(zs, ss, rank_major_outs, flat)
 
 
 class NF4LoRALinear(torch.autograd.Function):

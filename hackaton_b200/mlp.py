@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from .group import Projection, _refs, linear_backward_dx_group
-from .nf4 import _rows_view, _stream_ptr, _ws_buffers
+from .nf4 import _raw_stream, _rows_view, _stream_ptr, _ws_buffers
 
 _ws_need = {}
 
@@ -89,7 +89,7 @@ def _workspace(device, rows, cols, m, keep):
         _ws_need[key] = need
     if need == 0:
         return None, 0
-    skey = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    skey = (device.index, _raw_stream(device))
     buf = _ws_buffers.get(skey)
     if buf is None or buf.numel() < need:
         buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
@@ -172,7 +172,7 @@ def linear_backward_dx_swiglu(grad_out, down_w, gate, up):
         _ws_need[key] = need
     ws, ws_bytes = None, 0
     if need:
-        skey = (device.index, torch.cuda.current_stream(device).cuda_stream)
+        skey = (device.index, _raw_stream(device))
         buf = _ws_buffers.get(skey)
         if buf is None or buf.numel() < need:
             buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)

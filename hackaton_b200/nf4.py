@@ -42,9 +42,10 @@ def can_dequantize(packed, state):
             and getattr(state, "quant_type", None) == "nf4" and shape is not None
             and isinstance(absmax, torch.Tensor) and absmax.is_cuda
             and isinstance(code, torch.Tensor) and code.numel() == 16
-            and blocksize > 0 and blocksize % 8 == 0
-            and packed.numel() * 2 == _numel(shape) and _numel(shape) % 8 == 0
-            and _numel(shape) % blocksize == 0
+            and blocksize > 0 and blocksize % 8 == 0):
+        return False
+    numel = _numel(shape)
+    if not (packed.numel() * 2 == numel and numel % 8 == 0 and numel % blocksize == 0
             and packed.is_contiguous() and packed.data_ptr() % 4 == 0
             and getattr(state, "dtype", None) in _DTYPE_CODE):
         return False
@@ -101,6 +102,7 @@ class WeightRef:
             w.absmax = f32(state.absmax).data_ptr()
             w.nested_blocksize = 1
         self.struct = w
+        self.address = ctypes.addressof(w)
         self.keep = keep
         self.key = _content_key(packed, state)
         self.rows, self.cols = rows, cols
@@ -183,8 +185,14 @@ def weight_ref(packed, state) -> WeightRef:
     return ref
 
 
+def _raw_stream(device):
+    """Handle of the current stream (what torch.cuda.current_stream(device).cuda_stream says, without
+    building a stream object)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
 def _stream_ptr(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(_raw_stream(device))
 
 
 _ws_need = {}      # (device, n_rows, n_cols, m, backward) -> bytes of split-K scratch
@@ -195,6 +203,8 @@ def _workspace(device, n_rows, n_cols, m, backward):
     """Split-K scratch for one GEMM call on the current stream: (pointer, bytes) or (None, 0).
     One buffer per (device, stream), grown on demand; it needs no initialisation. Calls on the
     same stream run one after the other and can share it; other streams get their own."""
+    if m == 0:
+        return None, 0
     key = (device.index, n_rows, n_cols, m, backward)
     need = _ws_need.get(key)
     if need is None:
@@ -205,7 +215,12 @@ def _workspace(device, n_rows, n_cols, m, backward):
         _ws_need[key] = need
     if need == 0:
         return None, 0
-    skey = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    return _scratch(device, need)
+
+
+def _scratch(device, need):
+    """(pointer, bytes) of the current stream's buffer, grown to `need` bytes."""
+    skey = (device.index, _raw_stream(device))
     buf = _ws_buffers.get(skey)
     if buf is None or buf.numel() < need:
         buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
@@ -242,6 +257,11 @@ def _rows_view(t, cols):
     return t2
 
 
+def _rows(t):
+    """Number of rows of [..., cols]."""
+    return t.numel() // t.shape[-1]
+
+
 def linear_forward(x, packed, bias, state, xa=None, lora_b=None):
     """y = x . Wᵀ (+ bias) (+ xa . lora_bᵀ) through the fused kernel. x: fp16 [..., K]."""
     packed = packed.reshape(-1)
@@ -251,21 +271,8 @@ def linear_forward(x, packed, bias, state, xa=None, lora_b=None):
         raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {x.dtype}")
     if x.shape[-1] != ref.cols:
         raise ValueError(f"input has {x.shape[-1]} features, weight expects {ref.cols}")
-    x2 = _rows_view(x, ref.cols)
-    m = x2.shape[0]
-    y = torch.empty((m, ref.rows), dtype=torch.float16, device=x.device)
-    if m == 0:
-        return y.reshape(*x.shape[:-1], ref.rows)
-    if bias is not None:
-        bias = bias.to(torch.float16).contiguous()
-    ws, ws_bytes = _workspace(x.device, ref.rows, ref.cols, m, False)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().nf4b200_linear_fwd(
-            ctypes.byref(ref.struct), x2.data_ptr(), m, x2.stride(0),
-            None if bias is None else bias.data_ptr(),
-            None if xa is None else xa.data_ptr(), None if lora_b is None else lora_b.data_ptr(),
-            y.data_ptr(), y.stride(0), ws, ws_bytes, _stream_ptr(x.device)))
-    return y.reshape(*x.shape[:-1], ref.rows)
+    ws, ws_bytes = _workspace(x.device, ref.rows, ref.cols, _rows(x), False)
+    return _lib.host().linear_fwd(ref.address, x, bias, xa, lora_b, ws or 0, ws_bytes)
 
 
 def linear_backward_dx(grad_output, packed, state, u=None, lora_a=None):
@@ -275,18 +282,10 @@ def linear_backward_dx(grad_output, packed, state, u=None, lora_a=None):
     ref = weight_ref(packed, state).prepare()
     if grad_output.dtype != torch.float16:
         raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {grad_output.dtype}")
-    g2 = _rows_view(grad_output, ref.rows)
-    m = g2.shape[0]
-    dx = torch.empty((m, ref.cols), dtype=torch.float16, device=grad_output.device)
-    if m == 0:
-        return dx.reshape(*grad_output.shape[:-1], ref.cols)
-    ws, ws_bytes = _workspace(grad_output.device, ref.rows, ref.cols, m, True)
-    with torch.cuda.device(grad_output.device):
-        _lib.check(_lib.lib().nf4b200_linear_bwd_dx(
-            ctypes.byref(ref.struct), g2.data_ptr(), m, g2.stride(0),
-            None if u is None else u.data_ptr(), None if lora_a is None else lora_a.data_ptr(),
-            dx.data_ptr(), dx.stride(0), ws, ws_bytes, _stream_ptr(grad_output.device)))
-    return dx.reshape(*grad_output.shape[:-1], ref.cols)
+    if grad_output.shape[-1] != ref.rows:
+        raise ValueError(f"gradient has {grad_output.shape[-1]} features, weight gives {ref.rows}")
+    ws, ws_bytes = _workspace(grad_output.device, ref.rows, ref.cols, _rows(grad_output), True)
+    return _lib.host().linear_bwd_dx(ref.address, grad_output, u, lora_a, ws or 0, ws_bytes)
 
 
 class NF4Linear(torch.autograd.Function):

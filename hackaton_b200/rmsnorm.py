@@ -12,41 +12,19 @@ import torch
 
 from . import _lib
 from ._autograd import call
-from .nf4 import _stream_ptr
-
-
-def _out_code(dtype):
-    return _lib.F16 if dtype == torch.float16 else _lib.F32
 
 
 def launch_forward(x2, delta2, weight, eps, to_half):
     """One forward pass over rows of fp32 `x2` (+ fp16 `delta2`). Returns (normalised rows in fp16
     or fp32, 1/rms per row, the fp32 sum x2 + delta2 or None)."""
-    rows, hidden = x2.shape
-    device = x2.device
-    out = torch.empty((rows, hidden), dtype=torch.float16 if to_half else torch.float32, device=device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=device)
-    total = None if delta2 is None else torch.empty_like(x2)
-    with torch.cuda.device(device):
-        _lib.check(_lib.lib().nf4b200_rmsnorm_fwd(
-            x2.data_ptr(), None if delta2 is None else delta2.data_ptr(), weight.data_ptr(),
-            None if total is None else total.data_ptr(), out.data_ptr(), _out_code(out.dtype),
-            rstd.data_ptr(), rows, hidden, float(eps), _stream_ptr(device)))
-    return out, rstd, total
+    return _lib.host().rmsnorm_fwd(x2, delta2, weight, float(eps), to_half)
 
 
 def launch_backward(x2, weight, rstd, dy2, d_total=None, dx16=None):
     """Gradient with respect to the normalised rows' input; `d_total` (fp32, optional) is added in
     the same pass (the gradient that reached the sum directly), `dx16` (optional) a contiguous fp16
     tensor that receives the result's rounding."""
-    rows, hidden = x2.shape
-    dx = torch.empty_like(x2)
-    with torch.cuda.device(x2.device):
-        _lib.check(_lib.lib().nf4b200_add_rmsnorm_bwd(
-            x2.data_ptr(), weight.data_ptr(), rstd.data_ptr(), dy2.data_ptr(), _out_code(dy2.dtype),
-            None if d_total is None else d_total.data_ptr(), dx.data_ptr(),
-            None if dx16 is None else dx16.data_ptr(), rows, hidden, _stream_ptr(x2.device)))
-    return dx
+    return _lib.host().rmsnorm_bwd(x2, weight, rstd, dy2, d_total, dx16)
 
 
 def _rows(t):

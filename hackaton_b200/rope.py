@@ -56,30 +56,13 @@ class _RotateOp:
             raise TypeError(f"hackaton_b200: qkv_rotate takes fp16 or fp32 projections, got {q.dtype}")
         if cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.dim() != 3:
             raise TypeError("hackaton_b200: qkv_rotate takes fp32 cos / sin of shape (1 or B, T, D)")
-        cos, sin = cos.contiguous(), sin.contiguous()
-        geo = RotateGeometry(tokens=q.shape[0], seq=self.seq, heads=self.heads, kv_heads=self.kv_heads,
-                             dim=q.shape[-1] // self.heads, padded=self.padded,
-                             batch_stride=0 if cos.shape[0] == 1 else cos.stride(0),
-                             proj_dtype=q.dtype)
-        index = tuple(t.to(torch.int32).contiguous() for t in (b_idx, t_idx))
-        if self.padded:   # positions no token maps to stay zero
-            shape, make = (self.batch, self.heads, self.seq, geo.dim), torch.zeros
-        else:
-            shape, make = (geo.tokens, self.heads, geo.dim), torch.empty
-        heads_out = tuple(make(shape, dtype=torch.float16, device=q.device) for _ in range(3))
-        launch(tuple(t.contiguous() for t in (q, k, v)), heads_out, cos, sin, *index, geo, False)
-        keep(cos, sin, *index, geo=geo)
-        return heads_out
+        *heads_out, cos, sin, b_idx, t_idx, geo = _lib.host().rotate_fwd(
+            q, k, v, cos, sin, b_idx, t_idx, self.batch, self.seq, self.heads, self.kv_heads, self.padded)
+        keep(cos, sin, b_idx, t_idx, geo=geo)
+        return tuple(heads_out)
 
     def grad(self, kept, *head_grads):
-        cos, sin, b_idx, t_idx = kept.tensors
-        geo = kept.geo
-        src = tuple(g.to(torch.float16).contiguous() for g in head_grads)
-        widths = (geo.heads, geo.kv_heads, geo.kv_heads)
-        dst = tuple(torch.empty(geo.tokens, w * geo.dim, dtype=geo.proj_dtype, device=src[0].device)
-                    for w in widths)
-        launch(src, dst, cos, sin, b_idx, t_idx, geo, True)
-        return dst + (None, None, None, None)
+        return _lib.host().rotate_bwd(*head_grads, *kept.tensors, kept.geo) + (None, None, None, None)
 
 
 def qkv_rotate(q, k, v, cos, sin, b_idx, t_idx, batch, seq, heads, kv_heads, padded=False):

@@ -193,3 +193,43 @@ def test_sm_limit_keeps_results(cuda_lib):
     assert rel(y, nf4_oracle.linear_fwd(x, w)) <= TOL
     assert rel(dx, nf4_oracle.linear_bwd(dy, w)) <= TOL
     cuda_lib.device_status()
+
+
+def test_input_forms_of_the_calls(cuda_lib):
+    """Everything the linear calls take besides a contiguous [M, K] input: more and fewer dimensions,
+    strided, misaligned, transposed and broadcast rows, no rows, an fp32 bias; each equal to the call
+    on a contiguous copy, forward and backward, alone and as a group. Wrong widths are refused."""
+    from hackaton_b200.group import linear_backward_dx_group, linear_forward_group
+    from hackaton_b200.nf4 import linear_backward_dx, linear_forward
+
+    n, k = 256, 192
+    weights = [synthetic_weight(n, k, True, seed=i, device="cuda") for i in (1, 2)]
+    (packed, state), bias = weights[0], torch.randn(n, device="cuda")
+    big = torch.randn(6, 5, 2 * k + 16, device="cuda").half()
+    forms = {
+        "3-d": big[..., :k].contiguous(), "1-d": big[0, 0, :k].contiguous(), "strided": big[0, :, :k],
+        "misaligned": big[0, :, 3:3 + k], "transposed": torch.randn(k, 20, device="cuda").half().t(),
+        "broadcast": big[0, :1, :k].expand(7, k), "3-d strided": big[::2, :, 8:8 + k],
+        "no rows": big[:0, 0, :k], "one row": big[0, :1, 8:8 + k],
+    }
+    for name, x in forms.items():
+        plain = x.contiguous().clone()
+        y = linear_forward(x, packed, bias, state)
+        assert y.shape == (*x.shape[:-1], n) and y.is_contiguous(), name
+        assert torch.equal(y, linear_forward(plain, packed, bias.half(), state)), name
+        ys = linear_forward_group(x, weights, [bias, None])
+        assert [t.shape for t in ys] == [y.shape] * 2 and torch.equal(ys[0], y), name
+        at = 8 if y.numel() == n else 1    # (a single misaligned row counts as contiguous and is refused)
+        g = torch.randn(*x.shape[:-1], 2 * n, device="cuda").half()[..., at:n + at]
+        dx = linear_backward_dx(g, packed, state)
+        assert dx.shape == x.shape and torch.equal(dx, linear_backward_dx(g.contiguous().clone(), packed, state)), name
+        dx = linear_backward_dx_group([g, g], weights)
+        assert dx.shape == x.shape, name
+    for bad in (big[0, :, :k - 64], big[0, :, :2 * k]):
+        with pytest.raises((ValueError, RuntimeError)):
+            linear_forward(bad, packed, None, state)
+        with pytest.raises((ValueError, RuntimeError)):
+            linear_forward_group(bad, weights)
+    with pytest.raises((ValueError, RuntimeError)):
+        linear_forward(torch.randn(4, k).half(), packed, None, state)
+    assert cuda_lib.device_status() == 0
