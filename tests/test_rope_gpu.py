@@ -144,3 +144,36 @@ def test_backward_heads_of_128_vs_oracle(cuda_lib, heads, kv_heads, dtype):
         assert got.dtype == dtype
         torch.testing.assert_close(got.cpu().float(), ref.float(), **tol)
     cuda_lib.device_status()
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(12, 2, 128), (5, 1, 64), (6, 6, 256), (14, 2, 128), (28, 4, 128)])
+@pytest.mark.parametrize("tokens", [1, 37, 4200])     # both sides of the forward's CTAs-per-SM rule
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_heads_not_in_fours_and_copies_not_in_threes(cuda_lib, heads, kv_heads, dim, tokens, dtype):
+    """Item edges of the kernel (q heads in groups of four, copies in groups of three), per-batch cos /
+    sin tables, against 64-bit arithmetic; one rounding to the output type on top of fp32."""
+    from hackaton_b200.rope import qkv_rotate
+
+    g = torch.Generator(device="cuda").manual_seed(tokens + heads)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    seq, rep, half = 50, heads // kv_heads, dim // 2
+    at = torch.arange(tokens, device="cuda")
+    b, t = at // seq, at % seq
+    batch = (tokens + seq - 1) // seq
+    cos, sin = rand(batch, seq, dim), rand(batch, seq, dim)
+    ins = [rand(tokens, n * dim).to(dtype).requires_grad_() for n in (heads, kv_heads, kv_heads)]
+    outs = qkv_rotate(*ins, cos, sin, b, t, batch, seq, heads, kv_heads)
+    c, s = cos[b, t][:, None].double(), sin[b, t][:, None].double()
+    turn = lambda x: torch.cat((-x[..., half:], x[..., :half]), -1)  # noqa: E731
+    q, k, v = (x.detach().double().view(tokens, n, dim) for x, n in zip(ins, (heads, kv_heads, kv_heads)))
+    want = [q * c + turn(q) * s, (k * c + turn(k) * s).repeat_interleave(rep, 1), v.repeat_interleave(rep, 1)]
+    for o, w in zip(outs, want):
+        torch.testing.assert_close(o.double(), w, rtol=2.0 ** -10, atol=1e-3)
+    grads = [rand(*o.shape).half() for o in outs]
+    got = torch.autograd.grad(outs, ins, grads)
+    gq, gk, gv = (x.double() for x in grads)
+    gk, gv = (x.view(tokens, kv_heads, rep, dim).sum(2) for x in (gk, gv))
+    back = lambda x: (x * c - turn(x * s)).reshape(tokens, -1)  # noqa: E731
+    tol = dict(rtol=2.0 ** -10, atol=2e-3) if dtype == torch.float16 else dict(rtol=1e-5, atol=2e-5)
+    for o, w in zip(got, (back(gq), back(gk), gv.reshape(tokens, -1))):
+        torch.testing.assert_close(o.double(), w, **tol)
