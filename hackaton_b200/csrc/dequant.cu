@@ -7,8 +7,8 @@
 // value = table[code] * scale (fp32), rounded once to the output type.
 //
 // HBM bound: 0.5159 B read + 2 B written per weight (fp16 out, nested scales). One lane per
-// 32-bit word of codes (8 weights), eight words in flight per thread: 128-byte coalesced loads,
-// one wave of resident CTAs in a grid-stride loop. 16-bit outputs leave through a 32 KB staging
+// 32-bit word of codes (8 weights), several words in flight per thread: 128-byte coalesced loads.
+// 16-bit outputs: one wave of resident CTAs in a grid-stride loop; they leave through a 16 KB staging
 // area and one bulk copy per tile, fp32 outputs with 512-byte coalesced stores.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -61,7 +61,13 @@ struct Pack8<float> {
 };
 
 constexpr int DEQ_THREADS = 256;
-constexpr int DEQ_WORDS_PER_THREAD = 8;   // 32-bit code words (8 weights each) in flight per thread
+// 32-bit code words (8 weights each) in flight per thread. 16-bit outputs: four, so that eight CTAs with
+// their staging areas are resident (with eight words and six CTAs 8960 x 1536 took 7.9 us, now 7.2; 18944 x
+// 3584 bf16 38.5, now 36.2). fp32 outputs: eight, in CTAs of one tile (18944 x 3584: 73.3 us, 80.4 as one
+// wave of walking CTAs). The large ones are bound by writing: a plain fill of 136 MB takes 37.3 us and of
+// 272 MB 71.1 on this GPU (3.7 TB/s, against 6.5 for a copy's reads and writes together).
+template <bool STAGED>
+constexpr int deq_words = STAGED ? 4 : 8;
 
 // The 16-entry table is kept once per lane (entry e of lane l at [e * 32 + l]): every look-up of a
 // warp then goes to 32 different banks whatever the codes are.
@@ -78,7 +84,7 @@ __device__ __forceinline__ void bulk_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// STAGED (16-bit outputs): a tile is expanded into 32 KB of shared
+// STAGED (16-bit outputs): a tile is expanded into 16 KB of shared
 // memory and leaves as one bulk copy, so all that is left to do after the dependency wait is one
 // instruction per CTA.
 template <typename T, bool NESTED, bool SHIFTS, bool STAGED>
@@ -88,7 +94,8 @@ nf4_dequant_kernel(const uint32_t* __restrict__ codes, const void* __restrict__ 
                    const float* __restrict__ offset_ptr, const float* __restrict__ code16,
                    T* __restrict__ out, long long n_words, int words_per_block,
                    int nested_blocksize, int block_shift, int nested_shift) {
-    const long long tile = (long long)DEQ_THREADS * DEQ_WORDS_PER_THREAD;
+    constexpr int WORDS = deq_words<STAGED>;
+    const long long tile = (long long)DEQ_THREADS * WORDS;
     // Programmatic dependent launch: everything this kernel reads (codes, scales, tables) belongs
     // to the weight and is never written by a kernel of the stream, so the first tile's loads and
     // the table set-up run while the predecessor is still draining; the dependency wait comes
@@ -96,15 +103,15 @@ nf4_dequant_kernel(const uint32_t* __restrict__ codes, const void* __restrict__ 
     grid_dep_launch();
     __shared__ float table[16 * 32];
     __shared__ float table2[256];
-    __shared__ __align__(128) uint4 stage[STAGED ? DEQ_THREADS * DEQ_WORDS_PER_THREAD : 1];
+    __shared__ __align__(128) uint4 stage[STAGED ? DEQ_THREADS * WORDS : 1];
     const float* my_table = table + (threadIdx.x & 31);
 
-    uint32_t word[DEQ_WORDS_PER_THREAD];
-    float raw[DEQ_WORDS_PER_THREAD];      // flat: the scale; nested: the second-level scale
-    uint32_t q8[DEQ_WORDS_PER_THREAD];    // nested: the 8-bit first-level code
+    uint32_t word[WORDS];
+    float raw[WORDS];      // flat: the scale; nested: the second-level scale
+    uint32_t q8[WORDS];    // nested: the 8-bit first-level code
     auto issue = [&](long long base) {
 #pragma unroll
-        for (int j = 0; j < DEQ_WORDS_PER_THREAD; ++j) {
+        for (int j = 0; j < WORDS; ++j) {
             const long long w = base + j * DEQ_THREADS + threadIdx.x;
             word[j] = 0;
             raw[j] = 0.f;
@@ -138,7 +145,7 @@ nf4_dequant_kernel(const uint32_t* __restrict__ codes, const void* __restrict__ 
                 __syncthreads();
             }
 #pragma unroll
-            for (int j = 0; j < DEQ_WORDS_PER_THREAD; ++j) {
+            for (int j = 0; j < WORDS; ++j) {
                 const long long w = base + j * DEQ_THREADS + threadIdx.x;
                 if (w < n_words) {
                     const float scale = NESTED ? nested_scale(table2[q8[j]], raw[j], offset) : raw[j];
@@ -162,7 +169,7 @@ nf4_dequant_kernel(const uint32_t* __restrict__ codes, const void* __restrict__ 
         } else {
             if (!waited) { grid_dep_wait(); waited = true; }
 #pragma unroll
-            for (int j = 0; j < DEQ_WORDS_PER_THREAD; ++j) {
+            for (int j = 0; j < WORDS; ++j) {
                 const long long w = base + j * DEQ_THREADS + threadIdx.x;
                 if (w < n_words) {
                     const float scale = NESTED ? nested_scale(table2[q8[j]], raw[j], offset) : raw[j];
@@ -194,12 +201,10 @@ static int exact_log2(long long v) {
 template <typename T, bool STAGED>
 static cudaError_t launch_t(const DequantArgs& a, cudaStream_t stream) {
     const long long n_words = a.n / 8;
-    const long long tile = (long long)DEQ_THREADS * DEQ_WORDS_PER_THREAD;
+    const long long tile = (long long)DEQ_THREADS * deq_words<STAGED>;
     long long blocks = (n_words + tile - 1) / tile;
-    // One wave: as many CTAs as are resident at once (8 per SM at 256 threads, 6 with the 32 KB
-    // staging area), each walking the words in grid-stride order; a second, partly filled wave
-    // would cost as much as the first.
-    const long long cap = (long long)a.sm_count * (STAGED ? 6 : 8);
+    // 16-bit outputs: one wave, eight resident CTAs per SM walking the words in grid-stride order.
+    const long long cap = STAGED ? (long long)a.sm_count * 8 : 0x7FFFFFFFll;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     const int wpb = a.blocksize / 8;
