@@ -99,7 +99,7 @@ def _workspace(device, rows, cols, m, keep):
 
 def gate_up_swiglu_forward(x, gate_w, up_w, keep: bool):
     """gate_w, up_w: (packed, state). Returns (hidden, gate, up); gate and up are None unless
-    `keep`. One kernel for more than 256 token rows (see nf4b200_gate_up_swiglu_fwd)."""
+    `keep`. One kernel for more than 256 and for up to 32 token rows (see nf4b200_gate_up_swiglu_fwd)."""
     refs = _refs([gate_w, up_w])
     if refs[0].rows != refs[1].rows:
         raise ValueError("hackaton_b200: gate and up projections differ in shape")
