@@ -289,3 +289,20 @@ def test_mlp_patch_routes_and_falls_through(monkeypatch):
     monkeypatch.setattr(patches, "_eligible", lambda x, state, weight, bias: False)
     assert forward(block, x) == "original"
     assert len(calls) == 1
+
+
+def test_loss_chunks_cover_every_row_once():
+    """The row chunks of the lm_head loss: in order, without gaps, at most CHUNK_ROWS rows, whole GEMM
+    tiles except for the last, and never a last chunk that is short because the others are full."""
+    from hackaton_b200.lm_loss import CHUNK_ROWS, CHUNK_TILE, _chunks
+
+    assert _chunks(0) == []
+    for rows in [*range(1, 5200, 7), 2047, 2048, 2049, 4096, 4097, 6145, 100_000]:
+        parts = _chunks(rows)
+        sizes = [p.stop - p.start for p in parts]
+        assert parts[0].start == 0 and parts[-1].stop == rows
+        assert all(a.stop == b.start for a, b in zip(parts, parts[1:]))
+        assert max(sizes) <= CHUNK_ROWS and min(sizes) > 0
+        assert all(s % CHUNK_TILE == 0 for s in sizes[:-1])
+        assert len(parts) <= -(-rows // CHUNK_ROWS) + 1
+        assert sizes[-1] >= sizes[0] - len(parts) * CHUNK_TILE
