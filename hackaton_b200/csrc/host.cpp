@@ -156,6 +156,7 @@ lora_side(const std::vector<Tensor>& inputs, const std::vector<Tensor>& ps, cons
     std::vector<Tensor> keep, products, p16s, b16s;
     Opts b16ts;
     int64_t m = -1;
+    bool whole = true;   // every input in whole 16-byte pieces, as the side kernel reads it
     for (int i = 0; i < n; ++i) {
         const int64_t c = inputs[i].size(-1);
         const Tensor i2 = rows_view(inputs[i], c), p = factor(ps[i]);
@@ -165,6 +166,7 @@ lora_side(const std::vector<Tensor>& inputs, const std::vector<Tensor>& ps, cons
         TORCH_CHECK(i2.size(0) == m, "lora_side: inputs differ in their number of rows");
         nf4b200_lora_item& it = items[i];
         it.in = i2.const_data_ptr(); it.c = c; it.ld_in = i2.stride(0);
+        whole = whole && c % 8 == 0 && it.ld_in % 8 == 0 && (reinterpret_cast<uintptr_t>(it.in) & 15) == 0;
         it.p = p.const_data_ptr(); it.p_f32 = p.scalar_type() == at::kFloat;
         it.scaling = (float)scalings[i];
         products.push_back(at::empty({m, RANK}, options));
@@ -184,11 +186,14 @@ lora_side(const std::vector<Tensor>& inputs, const std::vector<Tensor>& ps, cons
         it.b16t = transpose ? b16ts.back()->data_ptr() : nullptr;
         keep.push_back(b);
     }
-    if (m == 0) {   // nothing to multiply: the copies and zeros by torch
+    if (m == 0 || !whole) {   // nothing to multiply, or columns that are not eights: copies and zeros by torch
         for (int i = 0; i < n; ++i) {
-            p16s[i].copy_(ps[i].detach());
+            if (items[i].p_f32) p16s[i].copy_(ps[i].detach());
+            if (m > 0)
+                check(nf4b200_lora_down(items[i].in, m, items[i].c, items[i].ld_in, p16s[i].const_data_ptr(),
+                                        items[i].c, 1, items[i].scaling, items[i].out, stream_of(inputs[0])));
             if (bs.empty()) continue;
-            b16s[i].copy_(bs[i].detach());
+            if (items[i].b_f32) b16s[i].copy_(bs[i].detach());
             if (transpose) b16ts[i]->copy_(bs[i].detach().t());
         }
         if (zero.has_value()) zero->zero_();

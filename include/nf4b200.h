@@ -234,7 +234,9 @@ int nf4b200_launches_group(int count, const int64_t* n_rows, int64_t n_cols, int
  *   drained; gate and up are rounded to fp16 first, so `hidden` holds what the two-step path
  *   gives. gate_out and up_out may both be NULL (inference: only `hidden` is written, half the
  *   output bytes of the plain grouped launch); training keeps them for the backward pass like
- *   the reference does. With fewer rows it runs the grouped GEMM and nf4b200_swiglu_fwd; scratch
+ *   the reference does. Up to 32 rows, with both scale tables and n_rows a multiple of 16, the
+ *   weight-streaming kernel forms the product where its partial sums meet, again from gate and up
+ *   rounded to fp16. Otherwise it runs the grouped GEMM and nf4b200_swiglu_fwd; scratch
  *   as nf4b200_gate_up_swiglu_workspace_bytes says (keep = 1 when gate_out / up_out are given).
  * nf4b200_swiglu_fwd / nf4b200_swiglu_bwd: the elementwise form on n contiguous fp16 values:
  *   hidden = gate * sigmoid(gate) * up;  d_up = d_hidden * gate * sig;

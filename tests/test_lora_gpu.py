@@ -141,3 +141,18 @@ def test_unmodified_when_only_b_needs_a_gradient(cuda_lib):
     grad, = torch.autograd.grad(y, b, gy)
     want = gy.double().t() @ (2.0 * x.double() @ a.half().double().t()).half().double()
     assert float((grad.double() - want).abs().max()) <= 1e-3 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("c,offset", [(100, 0), (64, 3), (20, 1)])
+def test_side_products_of_ragged_inputs(cuda_lib, c, offset):
+    """Columns or addresses in no whole 16-byte pieces (the gradient of a weight with such a number of
+    rows): the layout-agnostic product and copies by torch, same results."""
+    from hackaton_b200.lora import lora_side
+
+    x = torch.randn(12 * c + offset, device="cuda").half()[offset:].view(12, c)
+    p, b, zero = torch.randn(16, c, device="cuda"), torch.randn(24, 16, device="cuda"), torch.ones(64, device="cuda")
+    (o,), (p16,), (b16,), (bt,) = lora_side([x], [p], [0.5], [b], transpose=True, zero=zero)
+    want = 0.5 * x.double() @ p.half().double().t()
+    assert float((o.double() - want).abs().max()) <= 1e-3 * float(want.abs().max())
+    assert torch.equal(p16, p.half()) and torch.equal(b16, b.half()) and torch.equal(bt, b.half().t())
+    assert not zero.any()
