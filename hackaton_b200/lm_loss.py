@@ -16,12 +16,17 @@ from ._autograd import call
 from .dense import fp16_linear
 from .nf4 import _stream_ptr
 
-# Most rows of logits alive at a time. The reference holds 256 (solution/lm_loss.py:27) to fit 16 GB;
-# every chunk reads the whole head weight twice, so on a GPU with 180 GB more rows per chunk pay:
-# 2048 x 151,936 from 1536 takes 8 x 283 us in chunks of 256, 4 x 466 of 512, 2 x 864 of 1024 and
-# 1664 in one (622 MB of fp16 logits).
-CHUNK_ROWS = 2048
-CHUNK_TILE = 512      # token rows of the GEMM's largest tile
+# Rows of logits alive at a time: CHUNK_ROWS, halved while they would take more than LOGITS_BYTES or more
+# than there is, down to MIN_ROWS (the reference's number, solution/lm_loss.py:27). Every chunk reads the
+# whole head weight, so more rows pay: 2048 rows x 151,936 from 1536 features, both directions, 2247 us in
+# chunks of 512, 2128 of 1024, 2064 in one that holds twice the memory.
+CHUNK_ROWS = 1024
+MIN_ROWS = 256
+LOGITS_BYTES = 320 << 20
+# Rows of the gradient's product: one tile of the GEMM. With more, its plan cuts the contraction over the
+# vocabulary into fewer slices: longer chains of fp32 additions, and the error of d_hidden against 64 bits
+# grows (2048 x 3584: 6.45e-4 with 256 and 512 rows, 6.50e-4 with 1024, 6.68e-4 with 2048).
+CHUNK_TILE = 512
 GRAD_SCALE = 1024.0   # the chunk gradients are kept in fp16 at this scale (solution/lm_loss.py:28)
 
 
@@ -94,25 +99,42 @@ def fused_cross_entropy(logits, targets, denom, inplace_grad=False):
     return call(_LossFromLogits(bool(inplace_grad)), logits.contiguous(), targets, denom)
 
 
-def _head_products(hidden_rows, weight):
+def _head_products(hidden_rows, weight, logits):
     """The two matrix products of one chunk: logits = hidden_rows . weightᵀ, and, once the logits
     have been turned into their gradient, d_hidden = d_logits . weight. fp16 weights (the model's
     own lm_head) go through this library's tcgen05 kernel; other dtypes (a test in fp32) use
-    torch's matmul."""
+    torch's matmul. Returns the second one."""
     if hidden_rows.dtype == torch.float16 and weight.dtype == torch.float16:
-        return (fp16_linear(hidden_rows, weight),
-                lambda d_logits, out: fp16_linear(d_logits, weight, transposed=True, out=out))
-    return (torch.nn.functional.linear(hidden_rows, weight),
-            lambda d_logits, out: torch.mm(d_logits, weight, out=out))
+        fp16_linear(hidden_rows, weight, out=logits)
+        return lambda d_logits, out: fp16_linear(d_logits, weight, transposed=True, out=out)
+    torch.mm(hidden_rows, weight.t(), out=logits)
+    return lambda d_logits, out: torch.mm(d_logits, weight, out=out)
 
 
-def _chunks(rows):
-    """Row slices of at most CHUNK_ROWS rows, of about equal size (no short last one, which would
-    read the whole weight for a few rows), whole tiles except for the last."""
-    if rows == 0:
-        return []
-    count = -(-rows // CHUNK_ROWS)
-    step = min(CHUNK_ROWS, -(-rows // (count * CHUNK_TILE)) * CHUNK_TILE)
+def _chunk_rows(vocab, itemsize):
+    """Rows of (rows, vocab) logits that LOGITS_BYTES allows."""
+    rows = CHUNK_ROWS
+    while rows > MIN_ROWS and rows * vocab * itemsize > LOGITS_BYTES:
+        rows //= 2
+    return rows
+
+
+def _logits_buffer(rows, vocab, like):
+    """Room for the logits of a chunk of at most `rows` rows."""
+    step = _chunk_rows(vocab, like.element_size())
+    while True:
+        try:
+            return torch.empty(min(step, rows), vocab, dtype=like.dtype, device=like.device)
+        except torch.OutOfMemoryError:
+            if step <= MIN_ROWS:
+                raise
+            step //= 2
+
+
+def _chunks(rows, step=None):
+    """Row slices of `step` (CHUNK_ROWS) rows, the last one with what is left: few rows take the GEMM's
+    smaller tiles, so a short chunk costs less than chunks of equal size in part-filled tiles."""
+    step = step or CHUNK_ROWS
     return [slice(lo, min(lo + step, rows)) for lo in range(0, rows, step)]
 
 
@@ -131,12 +153,15 @@ class _HeadAndLoss:
         d_hidden = torch.empty_like(hidden)
         unit = torch.full((1,), GRAD_SCALE, dtype=torch.float32, device=device)
         with torch.autocast("cuda", enabled=False):
-            for rs in _chunks(rows):
-                logits, back = _head_products(hidden[rs], weight)
+            buffer = _logits_buffer(rows, weight.shape[0], hidden)
+            for rs in _chunks(rows, buffer.shape[0]):
+                logits = buffer[:rs.stop - rs.start]
+                back = _head_products(hidden[rs], weight, logits)
                 ce_stats(logits, targets[rs], True,
                          out=(stats["lse"][rs], stats["loss"][rs], stats["entropy"][rs], argmax[rs]))
                 ce_grad(logits, targets[rs], stats["lse"][rs], unit, logits)
-                back(logits, d_hidden[rs])
+                for part in _chunks(logits.shape[0], CHUNK_TILE):
+                    back(logits[part], d_hidden[rs][part])
         keep(d_hidden, denom)
         keep.constant(stats["loss"], stats["entropy"], argmax)
         return stats["loss"].sum() / denom, stats["loss"], stats["entropy"], argmax

@@ -292,17 +292,50 @@ def test_mlp_patch_routes_and_falls_through(monkeypatch):
 
 
 def test_loss_chunks_cover_every_row_once():
-    """The row chunks of the lm_head loss: in order, without gaps, at most CHUNK_ROWS rows, whole GEMM
-    tiles except for the last, and never a last chunk that is short because the others are full."""
+    """The row chunks of the lm_head loss: in order, without gaps, all full but the last."""
     from hackaton_b200.lm_loss import CHUNK_ROWS, CHUNK_TILE, _chunks
 
-    assert _chunks(0) == []
-    for rows in [*range(1, 5200, 7), 2047, 2048, 2049, 4096, 4097, 6145, 100_000]:
-        parts = _chunks(rows)
-        sizes = [p.stop - p.start for p in parts]
-        assert parts[0].start == 0 and parts[-1].stop == rows
-        assert all(a.stop == b.start for a, b in zip(parts, parts[1:]))
-        assert max(sizes) <= CHUNK_ROWS and min(sizes) > 0
-        assert all(s % CHUNK_TILE == 0 for s in sizes[:-1])
-        assert len(parts) <= -(-rows // CHUNK_ROWS) + 1
-        assert sizes[-1] >= sizes[0] - len(parts) * CHUNK_TILE
+    assert _chunks(0) == [] and CHUNK_ROWS % CHUNK_TILE == 0
+    for rows in [*range(1, 5200, 7), 2047, 2048, 2049, 4096, 4097, 6145, 8193, 100_000]:
+        for step in (CHUNK_ROWS, CHUNK_TILE, 256):
+            parts = _chunks(rows, step)
+            sizes = [p.stop - p.start for p in parts]
+            assert parts[0].start == 0 and parts[-1].stop == rows
+            assert all(a.stop == b.start for a, b in zip(parts, parts[1:]))
+            assert sizes[:-1] == [step] * (len(sizes) - 1) and 0 < sizes[-1] <= step
+        assert _chunks(rows) == _chunks(rows, CHUNK_ROWS)
+
+
+@pytest.mark.parametrize("vocab", [1000, 32_000, 151_936, 163_840, 163_848, 262_144, 1_000_000])
+@pytest.mark.parametrize("itemsize", [2, 4])
+def test_loss_chunks_bound_the_logits(vocab, itemsize):
+    """The logits alive at a time take at most LOGITS_BYTES, or what the reference's 256 rows take."""
+    from hackaton_b200.lm_loss import CHUNK_ROWS, LOGITS_BYTES, _chunk_rows
+
+    rows = _chunk_rows(vocab, itemsize)
+    assert 256 <= rows <= CHUNK_ROWS
+    assert rows * vocab * itemsize <= max(LOGITS_BYTES, 256 * vocab * itemsize)
+
+
+@pytest.mark.parametrize("most", [100, 255, 256, 700, 5000])
+def test_loss_takes_fewer_rows_where_memory_is_short(monkeypatch, most):
+    """An allocation that does not fit is tried with fewer rows, down to the reference's 256."""
+    from hackaton_b200 import lm_loss
+
+    real, asked = torch.empty, []
+
+    def empty(rows, cols, **kw):
+        asked.append(rows)
+        if rows > most:
+            raise torch.OutOfMemoryError("no room")
+        return real(rows, cols, **kw)
+
+    monkeypatch.setattr(lm_loss.torch, "empty", empty)
+    like = torch.zeros(1, dtype=torch.float16)
+    if most < 256:
+        with pytest.raises(torch.OutOfMemoryError):
+            lm_loss._logits_buffer(3000, 64, like)
+    else:
+        got = lm_loss._logits_buffer(3000, 64, like).shape[0]
+        assert 256 <= got <= most and got * 2 > min(most, lm_loss.CHUNK_ROWS)
+    assert asked[0] == lm_loss.CHUNK_ROWS and min(asked) >= 256

@@ -135,7 +135,7 @@ def test_thread_counts_and_segments(cuda_lib, rows, vocab, dtype):
 
 @pytest.mark.parametrize("rows", [2048, 2049, 2600])
 def test_chunks_cover_the_rows(cuda_lib, rows):
-    """Chunked against plain computation around the chunk limit (one chunk, two uneven ones)."""
+    """Chunked against plain computation around the chunk limit (whole chunks, a last one of one row, a part-filled one)."""
     from hackaton_b200.lm_loss import CHUNK_ROWS, _chunks, linear_cross_entropy
 
     parts = _chunks(rows)
@@ -153,3 +153,29 @@ def test_chunks_cover_the_rows(cuda_lib, rows):
     grad, = torch.autograd.grad(loss, hidden)
     torch.testing.assert_close(loss.double(), ref, rtol=1e-4, atol=1e-4)
     assert (grad.double() - want).norm() <= 5e-3 * want.norm()   # fp16 logits, gradients and sums
+
+
+@pytest.mark.parametrize("hidden_size", [1536, 3584])
+def test_chunk_size_does_not_move_the_gradient(cuda_lib, monkeypatch, hidden_size):
+    """The chunks in use give what the reference's 256 rows give, up to the order of the fp32 sums of
+    the softmax statistics (their 1e-6 moves a few fp16 roundings of the logits' gradient): 1e-5. With
+    more rows in the gradient's product its longer chains of fp32 additions make it 1e-4 to 2e-4."""
+    from hackaton_b200 import lm_loss
+
+    g = torch.Generator(device="cuda").manual_seed(hidden_size)
+    hidden = torch.randn(2560, hidden_size, device="cuda", generator=g).half().requires_grad_()
+    weight = (torch.randn(151_936, hidden_size, device="cuda", generator=g) * 0.04).half()
+    targets = torch.randint(0, 151_936, (2560,), device="cuda", generator=g)
+    denom = torch.tensor(2560.0, device="cuda")
+
+    def run():
+        loss, losses, entropy, argmax = lm_loss.linear_cross_entropy(hidden, weight, targets, denom)
+        return losses, argmax, torch.autograd.grad(loss, hidden)[0]
+
+    now = run()
+    monkeypatch.setattr(lm_loss, "CHUNK_ROWS", 256)
+    losses, argmax, grad = run()
+    assert torch.equal(now[1], argmax)
+    assert float((now[0] - losses).norm()) <= 1e-6 * float(losses.norm())
+    assert float((now[2].double() - grad.double()).norm()) <= 1e-5 * float(grad.double().norm())
+    cuda_lib.device_status()
