@@ -48,5 +48,5 @@ def fp16_linear(x, weight, transposed=False, bias=None, out=None):
         _lib.check(_lib.lib().nf4b200_fp16_linear(
             weight.data_ptr(), n, k, weight.stride(0), x2.data_ptr(), m, x2.stride(0),
             int(bool(transposed)), None if bias is None else bias.data_ptr(), y.data_ptr(),
-            y.stride(0), ws, ws_bytes, _stream_ptr(x.device)))
+            y.stride(0), None if ws is None else ws.data_ptr(), ws_bytes, _stream_ptr(x.device)))
     return y if out is not None else y.reshape(*x.shape[:-1], out_cols)

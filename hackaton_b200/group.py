@@ -83,7 +83,7 @@ def linear_forward_group(x, weights: Sequence, biases=None, xas=None, lora_bs=No
     ws, ws_bytes = _workspace(x.device, [r.rows for r in refs], cols, _rows(x), False)
     return _lib.host().linear_fwd_group(
         [r.address for r in refs], x, none if biases is None else list(biases), none if xas is None else list(xas),
-        none if lora_bs is None else list(lora_bs), ws or 0, ws_bytes)
+        none if lora_bs is None else list(lora_bs), ws, ws_bytes)
 
 
 def linear_backward_dx_group(grads: Sequence[torch.Tensor], weights: Sequence, us=None, lora_as=None):
@@ -97,7 +97,7 @@ def linear_backward_dx_group(grads: Sequence[torch.Tensor], weights: Sequence, u
             raise ValueError(f"gradient has {g.shape[-1]} features, weight gives {r.rows}")
     ws, ws_bytes = _workspace(grads[0].device, [r.rows for r in refs], refs[0].cols, _rows(grads[0]), True)
     return _lib.host().linear_bwd_dx_group([r.address for r in refs], list(grads), none if us is None else list(us),
-                                           none if lora_as is None else list(lora_as), ws or 0, ws_bytes)
+                                           none if lora_as is None else list(lora_as), ws, ws_bytes)
 
 
 class NF4LinearGroup(torch.autograd.Function):

@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from .group import Projection, _refs, linear_backward_dx_group
-from .nf4 import _raw_stream, _rows_view, _stream_ptr, _ws_buffers
+from .nf4 import _rows_view, _scratch, _stream_ptr
 
 _ws_need = {}
 
@@ -89,12 +89,7 @@ def _workspace(device, rows, cols, m, keep):
         _ws_need[key] = need
     if need == 0:
         return None, 0
-    skey = (device.index, _raw_stream(device))
-    buf = _ws_buffers.get(skey)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
-        _ws_buffers[skey] = buf
-    return buf.data_ptr(), need
+    return _scratch(device, need)
 
 
 def gate_up_swiglu_forward(x, gate_w, up_w, keep: bool):
@@ -118,8 +113,8 @@ def gate_up_swiglu_forward(x, gate_w, up_w, keep: bool):
             _lib.check(_lib.lib().nf4b200_gate_up_swiglu_fwd(
                 ctypes.byref(refs[0].struct), ctypes.byref(refs[1].struct), x2.data_ptr(), m,
                 x2.stride(0), None if gate is None else gate.data_ptr(),
-                None if up is None else up.data_ptr(), hidden.data_ptr(), ws, ws_bytes,
-                _stream_ptr(x.device)))
+                None if up is None else up.data_ptr(), hidden.data_ptr(),
+                None if ws is None else ws.data_ptr(), ws_bytes, _stream_ptr(x.device)))
     shape = (*lead, rows)
     return (hidden.reshape(shape), None if gate is None else gate.reshape(shape),
             None if up is None else up.reshape(shape))
@@ -170,18 +165,12 @@ def linear_backward_dx_swiglu(grad_out, down_w, gate, up):
         if need < 0:
             _lib.check(need)
         _ws_need[key] = need
-    ws, ws_bytes = None, 0
-    if need:
-        skey = (device.index, _raw_stream(device))
-        buf = _ws_buffers.get(skey)
-        if buf is None or buf.numel() < need:
-            buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
-            _ws_buffers[skey] = buf
-        ws, ws_bytes = buf.data_ptr(), need
+    ws, ws_bytes = _scratch(device, need) if need else (None, 0)
     with torch.cuda.device(device):
         _lib.check(_lib.lib().nf4b200_linear_bwd_dx_swiglu(
             ctypes.byref(ref.struct), g2.data_ptr(), m, g2.stride(0), gate.data_ptr(), up.data_ptr(),
-            d_gate.data_ptr(), d_up.data_ptr(), ws, ws_bytes, _stream_ptr(device)))
+            d_gate.data_ptr(), d_up.data_ptr(), None if ws is None else ws.data_ptr(), ws_bytes,
+            _stream_ptr(device)))
     return d_gate, d_up
 
 

@@ -196,13 +196,10 @@ def _stream_ptr(device):
 
 
 _ws_need = {}      # (device, n_rows, n_cols, m, backward) -> bytes of split-K scratch
-_ws_buffers = {}   # (device, stream) -> uint8 tensor
 
 
 def _workspace(device, n_rows, n_cols, m, backward):
-    """Split-K scratch for one GEMM call on the current stream: (pointer, bytes) or (None, 0).
-    One buffer per (device, stream), grown on demand; it needs no initialisation. Calls on the
-    same stream run one after the other and can share it; other streams get their own."""
+    """Split-K scratch for one GEMM call on the current stream: (buffer, bytes) or (None, 0)."""
     if m == 0:
         return None, 0
     key = (device.index, n_rows, n_cols, m, backward)
@@ -219,13 +216,12 @@ def _workspace(device, n_rows, n_cols, m, backward):
 
 
 def _scratch(device, need):
-    """(pointer, bytes) of the current stream's buffer, grown to `need` bytes."""
-    skey = (device.index, _raw_stream(device))
-    buf = _ws_buffers.get(skey)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
-        _ws_buffers[skey] = buf
-    return buf.data_ptr(), buf.numel()
+    """(buffer, bytes) for one call, uninitialised. Every call takes its own from torch's allocator and
+    drops it after the launch: the allocator hands it out again only behind the work of the stream it
+    was taken on, and a captured graph's lies in the graph's own pool for as long as the graph lives.
+    (A buffer kept per stream is neither: one that grows frees memory a captured graph still writes,
+    and two threads on a stream would interleave their launches on it.)"""
+    return _lib.host().scratch(need, device), need
 
 
 def _require(packed, state):
@@ -272,7 +268,7 @@ def linear_forward(x, packed, bias, state, xa=None, lora_b=None):
     if x.shape[-1] != ref.cols:
         raise ValueError(f"input has {x.shape[-1]} features, weight expects {ref.cols}")
     ws, ws_bytes = _workspace(x.device, ref.rows, ref.cols, _rows(x), False)
-    return _lib.host().linear_fwd(ref.address, x, bias, xa, lora_b, ws or 0, ws_bytes)
+    return _lib.host().linear_fwd(ref.address, x, bias, xa, lora_b, ws, ws_bytes)
 
 
 def linear_backward_dx(grad_output, packed, state, u=None, lora_a=None):
@@ -285,7 +281,7 @@ def linear_backward_dx(grad_output, packed, state, u=None, lora_a=None):
     if grad_output.shape[-1] != ref.rows:
         raise ValueError(f"gradient has {grad_output.shape[-1]} features, weight gives {ref.rows}")
     ws, ws_bytes = _workspace(grad_output.device, ref.rows, ref.cols, _rows(grad_output), True)
-    return _lib.host().linear_bwd_dx(ref.address, grad_output, u, lora_a, ws or 0, ws_bytes)
+    return _lib.host().linear_bwd_dx(ref.address, grad_output, u, lora_a, ws, ws_bytes)
 
 
 class NF4Linear(torch.autograd.Function):

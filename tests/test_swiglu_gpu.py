@@ -175,3 +175,38 @@ def test_whole_mlp_autograd(cuda_lib, m, hidden, inter):
     dx_ref = d_gate.float() @ w_gate.float() + d_up.float() @ w_up.float()
     assert nf4_oracle.max_rel_err(xg.grad.cpu(), dx_ref) <= TOL
     cuda_lib.device_status()
+
+
+def test_captured_graphs_keep_their_scratch(cuda_lib):
+    """A captured step writes its scratch (split-K planes, the two SwiGLU temporaries) on every replay:
+    that memory is the graph's own, whatever larger calls the same stream makes afterwards."""
+    from hackaton_b200 import Projection, nf4_swiglu_mlp
+    from hackaton_b200.nf4 import prepare_weights
+
+    weights = [synthetic_weight(n, k, True, seed=i, device="cuda")
+               for i, (n, k) in enumerate([(8960, 1536), (8960, 1536), (1536, 8960)])]
+    projs = [Projection(*w) for w in weights]
+    prepare_weights(weights)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    xs = [torch.randn(m, 1536, generator=g, device="cuda").half() for m in (40, 64, 256)]
+    stream, graphs, outs = torch.cuda.Stream(), [], []
+    torch.cuda.synchronize()
+    with torch.no_grad(), torch.cuda.stream(stream):
+        want = [nf4_swiglu_mlp(x, *projs).clone() for x in xs[:1]]
+        for x in xs[:2]:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                outs.append(nf4_swiglu_mlp(x, *projs))
+            graphs.append(graph)
+        want += [nf4_swiglu_mlp(x, *projs).clone() for x in xs[1:]]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        taken = [torch.full((size << 19,), 7.0, dtype=torch.float16, device="cuda")
+                 for size in (1, 2, 4, 6, 8, 12, 16, 24, 32) for _ in range(4)]
+    for graph, out, ref in zip(graphs, outs, want):
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+    assert all(bool((t == 7.0).all()) for t in taken)
+    cuda_lib.device_status()
