@@ -184,9 +184,8 @@ def query(device: int = 0) -> Props:
 def set_sm_limit(sms: int) -> None:
     """Caps the SMs the fused GEMM grids occupy (0 = all); see nf4b200_set_sm_limit."""
     check(lib().nf4b200_set_sm_limit(int(sms)))
-    from . import group, nf4     # scratch sizes were computed for the old grid
+    from . import nf4     # scratch sizes were computed for the old grid
     nf4._ws_need.clear()
-    group._ws_need.clear()
 
 
 def device_status() -> int:

@@ -13,7 +13,6 @@ which is exactly what autograd computes for such a fan-out, only with fewer and 
 
 from __future__ import annotations
 
-import ctypes
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -21,7 +20,7 @@ import torch
 
 from . import _lib
 from .lora import RANK, grad_buffer, lora_grad_batch, lora_side
-from .nf4 import _require, _rows, _scratch, weight_ref
+from .nf4 import _require, _rows, scratch_for, weight_ref
 
 MAX_GROUP = 4
 
@@ -37,24 +36,10 @@ class Projection:
     scaling: float = 1.0
 
 
-_ws_need = {}
-
-
 def _workspace(device, rows, cols, m, backward):
     if m == 0:
         return None, 0
-    key = (device.index, tuple(rows), cols, m, backward)
-    need = _ws_need.get(key)
-    if need is None:
-        arr = (ctypes.c_int64 * len(rows))(*rows)
-        with torch.cuda.device(device):
-            need = int(_lib.lib().nf4b200_workspace_bytes_group(len(rows), arr, cols, m, int(backward)))
-        if need < 0:
-            _lib.check(need)
-        _ws_need[key] = need
-    if need == 0:
-        return None, 0
-    return _scratch(device, need)
+    return scratch_for(device, "nf4b200_workspace_bytes_group", len(rows), tuple(rows), cols, m, int(backward))
 
 
 def _refs(items):

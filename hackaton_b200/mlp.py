@@ -20,9 +20,7 @@ import torch
 
 from . import _lib
 from .group import Projection, _refs, linear_backward_dx_group
-from .nf4 import _rows_view, _scratch, _stream_ptr
-
-_ws_need = {}
+from .nf4 import _rows_view, _stream_ptr, scratch_for
 
 
 def swiglu_forward(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
@@ -78,20 +76,6 @@ def silu_mul(gate, up):
     return SiluMul.apply(gate, up)
 
 
-def _workspace(device, rows, cols, m, keep):
-    key = (device.index, rows, cols, m, keep)
-    need = _ws_need.get(key)
-    if need is None:
-        with torch.cuda.device(device):
-            need = int(_lib.lib().nf4b200_gate_up_swiglu_workspace_bytes(rows, cols, m, int(keep)))
-        if need < 0:
-            _lib.check(need)
-        _ws_need[key] = need
-    if need == 0:
-        return None, 0
-    return _scratch(device, need)
-
-
 def gate_up_swiglu_forward(x, gate_w, up_w, keep: bool):
     """gate_w, up_w: (packed, state). Returns (hidden, gate, up); gate and up are None unless
     `keep`. One kernel for more than 256 and for up to 32 token rows (see nf4b200_gate_up_swiglu_fwd)."""
@@ -108,7 +92,7 @@ def gate_up_swiglu_forward(x, gate_w, up_w, keep: bool):
     gate = torch.empty_like(hidden) if keep else None
     up = torch.empty_like(hidden) if keep else None
     if m > 0:
-        ws, ws_bytes = _workspace(x.device, rows, cols, m, keep)
+        ws, ws_bytes = scratch_for(x.device, "nf4b200_gate_up_swiglu_workspace_bytes", rows, cols, m, int(keep))
         with torch.cuda.device(x.device):
             _lib.check(_lib.lib().nf4b200_gate_up_swiglu_fwd(
                 ctypes.byref(refs[0].struct), ctypes.byref(refs[1].struct), x2.data_ptr(), m,
@@ -157,15 +141,7 @@ def linear_backward_dx_swiglu(grad_out, down_w, gate, up):
     if m == 0:
         return d_gate, d_up
     device = g2.device
-    key = (device.index, "bwd", ref.rows, ref.cols, m)
-    need = _ws_need.get(key)
-    if need is None:
-        with torch.cuda.device(device):
-            need = int(_lib.lib().nf4b200_linear_bwd_dx_swiglu_workspace_bytes(ref.rows, ref.cols, m))
-        if need < 0:
-            _lib.check(need)
-        _ws_need[key] = need
-    ws, ws_bytes = _scratch(device, need) if need else (None, 0)
+    ws, ws_bytes = scratch_for(device, "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", ref.rows, ref.cols, m)
     with torch.cuda.device(device):
         _lib.check(_lib.lib().nf4b200_linear_bwd_dx_swiglu(
             ctypes.byref(ref.struct), g2.data_ptr(), m, g2.stride(0), gate.data_ptr(), up.data_ptr(),

@@ -195,24 +195,29 @@ def _stream_ptr(device):
     return ctypes.c_void_p(_raw_stream(device))
 
 
-_ws_need = {}      # (device, n_rows, n_cols, m, backward) -> bytes of split-K scratch
+_ws_need = {}      # (device, C function, its arguments) -> bytes of scratch under the SM limit in force
+
+
+def scratch_for(device, query, *sizes):
+    """(buffer, bytes) for a call on the current stream, or (None, 0). `query`: the C function that says
+    how much a call of these `sizes` (numbers, or tuples for arrays of them) takes."""
+    key = (device.index, query, sizes)
+    need = _ws_need.get(key)
+    if need is None:
+        args = [(ctypes.c_int64 * len(s))(*s) if isinstance(s, tuple) else s for s in sizes]
+        with torch.cuda.device(device):
+            need = int(getattr(_lib.lib(), query)(*args))
+        if need < 0:
+            _lib.check(need)
+        _ws_need[key] = need
+    return _scratch(device, need) if need else (None, 0)
 
 
 def _workspace(device, n_rows, n_cols, m, backward):
     """Split-K scratch for one GEMM call on the current stream: (buffer, bytes) or (None, 0)."""
     if m == 0:
         return None, 0
-    key = (device.index, n_rows, n_cols, m, backward)
-    need = _ws_need.get(key)
-    if need is None:
-        with torch.cuda.device(device):
-            need = int(_lib.lib().nf4b200_workspace_bytes(n_rows, n_cols, m, int(backward)))
-        if need < 0:
-            _lib.check(need)
-        _ws_need[key] = need
-    if need == 0:
-        return None, 0
-    return _scratch(device, need)
+    return scratch_for(device, "nf4b200_workspace_bytes", n_rows, n_cols, m, int(backward))
 
 
 def _scratch(device, need):

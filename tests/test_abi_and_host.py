@@ -339,3 +339,32 @@ def test_loss_takes_fewer_rows_where_memory_is_short(monkeypatch, most):
         got = lm_loss._logits_buffer(3000, 64, like).shape[0]
         assert 256 <= got <= most and got * 2 > min(most, lm_loss.CHUNK_ROWS)
     assert asked[0] == lm_loss.CHUNK_ROWS and min(asked) >= 256
+
+
+def test_sm_limit_drops_every_scratch_size(monkeypatch):
+    """Scratch sizes follow the SM limit: what was asked under one limit is asked again under another,
+    for every kind of call."""
+    from hackaton_b200 import _lib, group, mlp, nf4
+
+    asked = []
+
+    class Library:
+        def __getattr__(self, name):
+            return lambda *args: asked.append(name) or (0 if name == "nf4b200_set_sm_limit" else 256)
+
+    monkeypatch.setattr(_lib, "lib", Library)
+    monkeypatch.setattr(nf4, "_ws_need", {})
+    monkeypatch.setattr(nf4, "_scratch", lambda device, need: (None, need))
+    monkeypatch.setattr(nf4.torch.cuda, "device", lambda d: __import__("contextlib").nullcontext())
+    device = torch.device("cuda", 0)
+    calls = [lambda: nf4._workspace(device, 64, 64, 4, False), lambda: nf4._workspace(device, 64, 64, 4, True),
+             lambda: group._workspace(device, [64, 64], 64, 4, False),
+             lambda: mlp.scratch_for(device, "nf4b200_gate_up_swiglu_workspace_bytes", 64, 64, 4, 1),
+             lambda: mlp.scratch_for(device, "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", 64, 64, 4)]
+    for _ in range(2):
+        assert all(call()[1] == 256 for call in calls)
+    assert len(asked) == len(calls)
+    _lib.set_sm_limit(8)
+    assert all(call()[1] == 256 for call in calls)
+    assert len(asked) == 2 * len(calls) + 1
+    assert all(not hasattr(module, "_ws_need") for module in (group, mlp))

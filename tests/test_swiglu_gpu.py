@@ -210,3 +210,32 @@ def test_captured_graphs_keep_their_scratch(cuda_lib):
         assert torch.equal(out, ref)
     assert all(bool((t == 7.0).all()) for t in taken)
     cuda_lib.device_status()
+
+
+@pytest.mark.parametrize("m", [40, 200, 300])
+def test_scratch_follows_the_sm_limit(cuda_lib, m):
+    """A shape first seen under an SM limit, whose plan takes fewer K-slices, runs with all SMs again:
+    forward with and without kept activations, and backward."""
+    from hackaton_b200 import Projection, nf4_swiglu_mlp
+
+    weights = [synthetic_weight(n, k, True, seed=i, device="cuda")
+               for i, (n, k) in enumerate([(896, 512), (896, 512), (512, 896)])]
+    projs = [Projection(*w) for w in weights]
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn(m, 512, generator=g, device="cuda").half().requires_grad_()
+    dy = torch.randn(m, 512, generator=g, device="cuda").half()
+
+    def run():
+        with torch.no_grad():
+            plain = nf4_swiglu_mlp(x, *projs)
+        y = nf4_swiglu_mlp(x, *projs)
+        return plain, y.detach(), torch.autograd.grad(y, x, dy)[0]
+
+    try:
+        cuda_lib.set_sm_limit(4)
+        limited = run()
+    finally:
+        cuda_lib.set_sm_limit(0)
+    for a, b in zip(limited, run()):   # other slices: the order of the fp32 sums, then fp16 roundings
+        assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm())
+    cuda_lib.device_status()
