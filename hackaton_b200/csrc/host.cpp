@@ -38,6 +38,22 @@ void* raw(const Opt& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 
 const nf4b200_weight* weight(int64_t address) { return reinterpret_cast<const nf4b200_weight*>(address); }
 
+// Where the tensors of a weight lie and how often each has been written (inference tensors do not count
+// that), in a form that compares as a whole.
+py::bytes stamps(const Tensor& packed, const Tensor& absmax, const Tensor& code, const Opt& absmax2, const Opt& code2,
+                 const Opt& offset) {
+    const Tensor none;
+    const Tensor* all[] = {&packed, &absmax, &code, absmax2 ? &*absmax2 : &none, code2 ? &*code2 : &none,
+                           offset ? &*offset : &none};
+    int64_t r[12];
+    int n = 0;
+    for (const Tensor* t : all) {
+        r[n++] = t->defined() ? reinterpret_cast<int64_t>(t->const_data_ptr()) : 0;
+        r[n++] = t->defined() && !t->is_inference() ? t->_version() : -1;
+    }
+    return py::bytes(reinterpret_cast<const char*>(r), sizeof r);
+}
+
 // [..., cols] -> 2-D view with contiguous rows, 16-byte aligned and 8 elements apart (copied only if the
 // layout forces it).
 Tensor rows_view(const Tensor& t, int64_t cols) {
@@ -323,6 +339,7 @@ std::tuple<Tensor, Tensor, Tensor> rotate_bwd(const Tensor& gq, const Tensor& gk
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+    m.def("stamps", &stamps);
     m.def("scratch", &scratch);
     m.def("linear_fwd", &linear_fwd);
     m.def("linear_bwd_dx", &linear_bwd_dx);

@@ -69,13 +69,15 @@ class WeightRef:
 
     def __init__(self, packed, state):
         device = packed.device
+        key = _content_key(packed, state)   # (before anything is read)
         rows, cols = (int(state.shape[0]), int(state.shape[1])) if len(state.shape) == 2 else \
             (1, _numel(state.shape))
-        keep = [packed]
+        keep = [packed, state.absmax]
 
         def f32(t):
             if not isinstance(t, torch.Tensor):
                 t = torch.tensor(float(t))
+            keep.append(t)
             t = t.detach()
             if t.device != device or t.dtype != torch.float32 or not t.is_contiguous():
                 t = t.to(device=device, dtype=torch.float32).contiguous()
@@ -104,7 +106,7 @@ class WeightRef:
         self.struct = w
         self.address = ctypes.addressof(w)
         self.keep = keep
-        self.key = _content_key(packed, state)
+        self.key = key
         self.rows, self.cols = rows, cols
         self.scales16 = None
         self._ready = None   # (event, stream) of the table's construction while it may be pending
@@ -150,18 +152,18 @@ class WeightRef:
 
 
 def _content_key(packed, state):
-    """Identity of a weight's contents: where its tensors live and how often they have been
-    written in place. Loading other weights into the same storage (`copy_`, a second checkpoint)
-    bumps the version counters, so a cached descriptor (and its scale table) is not reused."""
-    nested = bool(getattr(state, "nested", False))
-    parts = [packed.data_ptr(), packed._version, state.absmax.data_ptr(), state.absmax._version,
-             nested]
-    if nested:
-        state2 = state.state2
-        offset = state.offset
-        parts += [state2.absmax.data_ptr(), state2.absmax._version,
-                  offset._version if isinstance(offset, torch.Tensor) else float(offset)]
-    return tuple(parts)
+    """Identity of everything a descriptor and its scale table are made from: where the tensors live,
+    how often they have been written in place, and the sizes. Loading other weights into the same
+    storage (`copy_`, a second checkpoint) bumps the version counters, another tensor in a field has
+    another address (the descriptor keeps the ones it was made from alive), so a cached descriptor is
+    not reused for either."""
+    stamps = _lib.host().stamps
+    if not getattr(state, "nested", False):
+        return stamps(packed, state.absmax, state.code, None, None, None), tuple(state.shape), state.blocksize
+    state2, offset = state.state2, state.offset
+    number = None if isinstance(offset, torch.Tensor) else float(offset)
+    return (stamps(packed, state.absmax, state.code, state2.absmax, state2.code, offset if number is None else None),
+            tuple(state.shape), state.blocksize, state2.blocksize, number)
 
 
 def prepare_weights(weights):

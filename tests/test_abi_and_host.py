@@ -368,3 +368,37 @@ def test_sm_limit_drops_every_scratch_size(monkeypatch):
     assert all(call()[1] == 256 for call in calls)
     assert len(asked) == 2 * len(calls) + 1
     assert all(not hasattr(module, "_ws_need") for module in (group, mlp))
+
+
+def test_weight_key_covers_what_the_descriptor_is_made_from():
+    """Every tensor and size that a descriptor or its scale table depends on changes the key, replaced
+    or written in place; a state nobody touched keeps it; inference tensors are taken."""
+    from hackaton_b200.nf4 import _content_key
+    from tests.util import synthetic_weight
+
+    def changes(state):
+        for owner in (state, state.state2):
+            for field in ("absmax", "code"):
+                t = getattr(owner, field)
+                yield lambda t=t: t.mul_(1)
+                yield lambda owner=owner, field=field, t=t: setattr(owner, field, t.clone())
+            yield lambda owner=owner: setattr(owner, "blocksize", owner.blocksize * 2)
+        yield lambda: state.offset.mul_(1)
+        yield lambda: setattr(state, "offset", state.offset.clone())
+        yield lambda: setattr(state, "offset", 0.25)
+        yield lambda: setattr(state, "shape", tuple(reversed(state.shape)))
+
+    packed, state = synthetic_weight(32, 128, True)
+    seen = [_content_key(packed, state)]
+    kept = []   # (a freed tensor's address could come back)
+    for change in changes(state):
+        kept.append((state.absmax, state.code, state.state2.absmax, state.state2.code, state.offset))
+        change()
+        seen.append(_content_key(packed, state))
+        assert seen[-1] == _content_key(packed, state)
+    packed.add_(0)
+    seen.append(_content_key(packed, state))
+    assert len(set(seen)) == len(seen)
+    with torch.inference_mode():
+        packed, state = synthetic_weight(32, 128, True)
+    assert _content_key(packed, state) == _content_key(packed, state)

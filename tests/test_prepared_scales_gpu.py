@@ -128,3 +128,47 @@ def test_group_without_tables(gather_only):
     dx = linear_backward_dx_group(dys, ws)
     want = sum(nf4.linear_backward_dx(d, p, s).float() for d, (p, s) in zip(dys, ws))
     assert (dx.float() - want).abs().max() <= 2e-2 * want.abs().max()
+
+
+def _swaps():
+    """What a program may do to a state between two calls: other tables, offsets, scales or codes, as new
+    tensors or written in place."""
+    def replace(owner, field, change):
+        return lambda packed, state: setattr(owner(state), field, change(getattr(owner(state), field)))
+
+    def write(owner, field, change):
+        return lambda packed, state: getattr(owner(state), field).copy_(change(getattr(owner(state), field)))
+
+    top, second = (lambda s: s), (lambda s: s.state2)
+    flip = lambda t: t.flip(0).contiguous()             # noqa: E731
+    half = lambda t: t * 0.5                            # noqa: E731
+    return {
+        "code replaced": replace(top, "code", flip), "code written": write(top, "code", flip),
+        "code2 replaced": replace(second, "code", flip), "code2 written": write(second, "code", flip),
+        "absmax2 replaced": replace(second, "absmax", half), "absmax2 written": write(second, "absmax", half),
+        "offset replaced": replace(top, "offset", half), "offset written": write(top, "offset", half),
+        "offset as a number": replace(top, "offset", lambda t: 2.0 * float(t)),
+        "absmax replaced": replace(top, "absmax", flip), "absmax written": write(top, "absmax", flip),
+        "packed written": lambda packed, state: packed.copy_(packed.flip(0)),
+    }
+
+
+@pytest.mark.parametrize("m", [4, 300])
+@pytest.mark.parametrize("swap", sorted(_swaps()))
+def test_a_changed_state_is_seen(cuda_lib, swap, m):
+    """A call after a change gives what a state that never was anything else gives."""
+    from hackaton_b200.nf4 import dequantize_nf4, linear_forward
+    from hackaton_b200.quantize import NestedState, QuantState
+
+    packed, state = synthetic_weight(128, 192, True, seed=3, device="cuda")
+    x = torch.randn(m, 192, generator=torch.Generator(device="cuda").manual_seed(m), device="cuda").half()
+    first = linear_forward(x, packed, None, state)
+    _swaps()[swap](packed, state)
+    fresh = QuantState(absmax=state.absmax.clone(), code=state.code.clone(), shape=state.shape,
+                       dtype=state.dtype, blocksize=state.blocksize, nested=True, offset=state.offset,
+                       state2=NestedState(state.state2.absmax.clone(), state.state2.code.clone(),
+                                          state.state2.blocksize))
+    y = linear_forward(x, packed, None, state)
+    assert torch.equal(y, linear_forward(x, packed.clone(), None, fresh)) and not torch.equal(y, first)
+    assert torch.equal(dequantize_nf4(packed, state), dequantize_nf4(packed.clone(), fresh))
+    cuda_lib.device_status()
