@@ -24,9 +24,10 @@ namespace {
 constexpr int64_t RANK = 16;
 constexpr int MAX_GROUP = 4, MAX_BATCH = 8;
 
-// A non-zero status becomes the package's own exception.
+// A non-zero status becomes the package's own exception. (The calls run without the interpreter lock.)
 void check(int rc) {
     if (rc == 0) return;
+    const py::gil_scoped_acquire lock;
     py::module_::import("hackaton_b200._lib").attr("check")(rc);
 }
 
@@ -306,9 +307,10 @@ void rotate(const Rotation& r, const Tensor (&src)[3], Tensor (&dst)[3], const T
 }
 
 // (q, k, v heads, and what the gradient needs: cos, sin, b_idx, t_idx as the kernel read them, geometry)
-py::tuple rotate_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos_in, const Tensor& sin_in,
-                     const Tensor& b_in, const Tensor& t_in, int64_t batch, int64_t seq, int64_t heads,
-                     int64_t kv_heads, bool padded) {
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Rotation>
+rotate_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos_in, const Tensor& sin_in,
+           const Tensor& b_in, const Tensor& t_in, int64_t batch, int64_t seq, int64_t heads, int64_t kv_heads,
+           bool padded) {
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor cos = cos_in.contiguous(), sin = sin_in.contiguous();
     const Tensor b_idx = b_in.to(at::kInt).contiguous(), t_idx = t_in.to(at::kInt).contiguous();
@@ -320,7 +322,7 @@ py::tuple rotate_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     for (auto& d : dst)   // padded: positions no token maps to stay zero
         d = padded ? at::zeros({batch, heads, seq, r.dim}, options) : at::empty({r.tokens, heads, r.dim}, options);
     rotate(r, src, dst, cos, sin, b_idx, t_idx, false);
-    return py::make_tuple(dst[0], dst[1], dst[2], cos, sin, b_idx, t_idx, r);
+    return {dst[0], dst[1], dst[2], cos, sin, b_idx, t_idx, r};
 }
 
 std::tuple<Tensor, Tensor, Tensor> rotate_bwd(const Tensor& gq, const Tensor& gk, const Tensor& gv, const Tensor& cos,
@@ -339,17 +341,19 @@ std::tuple<Tensor, Tensor, Tensor> rotate_bwd(const Tensor& gq, const Tensor& gk
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
-    m.def("stamps", &stamps);
-    m.def("scratch", &scratch);
-    m.def("linear_fwd", &linear_fwd);
-    m.def("linear_bwd_dx", &linear_bwd_dx);
-    m.def("linear_fwd_group", &linear_fwd_group);
-    m.def("linear_bwd_dx_group", &linear_bwd_dx_group);
-    m.def("lora_side", &lora_side);
-    m.def("lora_grad_batch", &lora_grad_batch);
-    m.def("rmsnorm_fwd", &rmsnorm_fwd);
-    m.def("rmsnorm_bwd", &rmsnorm_bwd);
     py::class_<Rotation>(m, "Rotation");
-    m.def("rotate_fwd", &rotate_fwd);
-    m.def("rotate_bwd", &rotate_bwd);
+    m.def("stamps", &stamps);
+    // An allocation or a launch can block (cudaMalloc, a full launch queue): other Python threads go on.
+    using unlocked = py::call_guard<py::gil_scoped_release>;
+    m.def("scratch", &scratch, unlocked());
+    m.def("linear_fwd", &linear_fwd, unlocked());
+    m.def("linear_bwd_dx", &linear_bwd_dx, unlocked());
+    m.def("linear_fwd_group", &linear_fwd_group, unlocked());
+    m.def("linear_bwd_dx_group", &linear_bwd_dx_group, unlocked());
+    m.def("lora_side", &lora_side, unlocked());
+    m.def("lora_grad_batch", &lora_grad_batch, unlocked());
+    m.def("rmsnorm_fwd", &rmsnorm_fwd, unlocked());
+    m.def("rmsnorm_bwd", &rmsnorm_bwd, unlocked());
+    m.def("rotate_fwd", &rotate_fwd, unlocked());
+    m.def("rotate_bwd", &rotate_bwd, unlocked());
 }
