@@ -310,11 +310,11 @@ void rotate(const Rotation& r, const Tensor (&src)[3], Tensor (&dst)[3], const T
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Rotation>
 rotate_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos_in, const Tensor& sin_in,
            const Tensor& b_in, const Tensor& t_in, int64_t batch, int64_t seq, int64_t heads, int64_t kv_heads,
-           bool padded) {
+           int64_t dim, bool padded) {
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor cos = cos_in.contiguous(), sin = sin_in.contiguous();
     const Tensor b_idx = b_in.to(at::kInt).contiguous(), t_idx = t_in.to(at::kInt).contiguous();
-    Rotation r = {q.size(0), seq, heads, kv_heads, q.size(-1) / heads, cos.size(0) == 1 ? 0 : cos.stride(0), padded,
+    Rotation r = {q.size(0), seq, heads, kv_heads, dim, cos.size(0) == 1 ? 0 : cos.stride(0), padded,
                   q.scalar_type() == at::kFloat};
     const Tensor src[3] = {q.contiguous(), k.contiguous(), v.contiguous()};
     const auto options = q.options().dtype(at::kHalf);

@@ -57,7 +57,8 @@ class _RotateOp:
         if cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.dim() != 3:
             raise TypeError("hackaton_b200: qkv_rotate takes fp32 cos / sin of shape (1 or B, T, D)")
         *heads_out, cos, sin, b_idx, t_idx, geo = _lib.host().rotate_fwd(
-            q, k, v, cos, sin, b_idx, t_idx, self.batch, self.seq, self.heads, self.kv_heads, self.padded)
+            q, k, v, cos, sin, b_idx, t_idx, self.batch, self.seq, self.heads, self.kv_heads,
+            q.shape[-1] // self.heads, self.padded)
         keep(cos, sin, b_idx, t_idx, geo=geo)
         return tuple(heads_out)
 

@@ -402,3 +402,20 @@ def test_weight_key_covers_what_the_descriptor_is_made_from():
     with torch.inference_mode():
         packed, state = synthetic_weight(32, 128, True)
     assert _content_key(packed, state) == _content_key(packed, state)
+
+
+def test_rotation_without_heads_is_an_error(monkeypatch):
+    """No query heads: Python's ZeroDivisionError, before any native code divides by it."""
+    from hackaton_b200 import _lib
+    from hackaton_b200.rope import _RotateOp
+
+    calls = []
+    host = types.SimpleNamespace(rotate_fwd=lambda *args: calls.append(args) or (None,) * 8)
+    monkeypatch.setattr(_lib, "host", lambda: host)
+    q = types.SimpleNamespace(is_cuda=True, dtype=torch.float16, shape=(4, 256))
+    table = torch.zeros(1, 4, 128)
+    with pytest.raises(ZeroDivisionError):
+        _RotateOp(1, 4, 0, 1, False).run(lambda *a, **k: None, q, q, q, table, table, None, None)
+    assert not calls
+    _RotateOp(1, 4, 2, 1, False).run(lambda *a, **k: None, q, q, q, table, table, None, None)
+    assert calls[0][7:] == (1, 4, 2, 1, 128, False)
