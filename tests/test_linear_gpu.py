@@ -211,6 +211,13 @@ def test_input_forms_of_the_calls(cuda_lib):
         "misaligned": big[0, :, 3:3 + k], "transposed": torch.randn(k, 20, device="cuda").half().t(),
         "broadcast": big[0, :1, :k].expand(7, k), "3-d strided": big[::2, :, 8:8 + k],
         "no rows": big[:0, 0, :k], "one row": big[0, :1, 8:8 + k],
+        "contiguous at an odd address": big.flatten()[1:1 + 5 * k].view(5, k),
+        "one row at an odd address": big.flatten()[3:3 + k].view(1, k),
+        "one row of an odd stride": big.flatten()[8:].as_strided((1, k), (k + 3, 1)),
+    }
+    outs = {
+        "strided": lambda g: g[..., 8:8 + n], "misaligned": lambda g: g[..., 1:1 + n],
+        "contiguous at an odd address": lambda g: g.flatten()[1:1 + g.numel() // 2].view(*g.shape[:-1], n),
     }
     for name, x in forms.items():
         plain = x.contiguous().clone()
@@ -219,12 +226,18 @@ def test_input_forms_of_the_calls(cuda_lib):
         assert torch.equal(y, linear_forward(plain, packed, bias.half(), state)), name
         ys = linear_forward_group(x, weights, [bias, None])
         assert [t.shape for t in ys] == [y.shape] * 2 and torch.equal(ys[0], y), name
-        at = 8 if y.numel() == n else 1    # (a single misaligned row counts as contiguous and is refused)
-        g = torch.randn(*x.shape[:-1], 2 * n, device="cuda").half()[..., at:n + at]
-        dx = linear_backward_dx(g, packed, state)
-        assert dx.shape == x.shape and torch.equal(dx, linear_backward_dx(g.contiguous().clone(), packed, state)), name
-        dx = linear_backward_dx_group([g, g], weights)
-        assert dx.shape == x.shape, name
+        wide = torch.randn(*x.shape[:-1], 2 * n, device="cuda").half()
+        for form, take in outs.items():
+            g = take(wide) if y.numel() else wide[..., :n]
+            copy = g.contiguous().clone()
+            dx = linear_backward_dx(g, packed, state)
+            assert dx.shape == x.shape and torch.equal(dx, linear_backward_dx(copy, packed, state)), (name, form)
+            both = linear_backward_dx_group([g, g], weights)
+            assert both.shape == x.shape, (name, form)
+            assert torch.equal(both, linear_backward_dx_group([copy, copy], weights)), (name, form)
+            if y.numel():    # two fp16 roundings and the sum of one fp16 result each
+                ref = dx.double() + linear_backward_dx(copy, *weights[1]).double()
+                assert float((both.double() - ref).norm()) <= 2e-3 * float(ref.norm()), (name, form)
     for bad in (big[0, :, :k - 64], big[0, :, :2 * k]):
         with pytest.raises((ValueError, RuntimeError)):
             linear_forward(bad, packed, None, state)
