@@ -119,7 +119,9 @@ constexpr uint32_t PAIR_AT = 2048;
 
 __device__ __forceinline__ uint32_t pair_lookup(uint32_t offset) {
     uint32_t v;
-    asm("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(offset), "n"(PAIR_AT));
+    // (volatile: the table is written again when a CTA walks on to another member, so a value is only good
+    // on this side of the barriers around that)
+    asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(offset), "n"(PAIR_AT));
     return v;
 }
 
