@@ -160,12 +160,17 @@ def host():
     global _host_module
     if _host_module is None:
         lib()
+        from .build import host_target
+
+        advice = "build it with `python -m hackaton_b200.build` (needs nvcc and g++)"
         try:
             from . import _host
         except ImportError as e:
-            raise RuntimeError(
-                "hackaton_b200/_host.so is missing or does not fit the installed torch: build it with "
-                "`python -m hackaton_b200.build` (needs nvcc and g++)") from e
+            raise RuntimeError("hackaton_b200/_host.so is missing or does not fit the installed torch: "
+                               + advice) from e
+        if _host.built_for != host_target():
+            raise RuntimeError(f"hackaton_b200/_host.so was built for {_host.built_for}, this is "
+                               f"{host_target()}: {advice}")
         _host_module = _host
     return _host_module
 

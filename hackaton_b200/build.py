@@ -45,18 +45,33 @@ def _stale() -> bool:
     return any(p.stat().st_mtime > built for p in deps)
 
 
+def host_target() -> str:
+    """What _host.so is built for, as it stands in the file and in its attribute `built_for`."""
+    import torch
+
+    return f"torch {torch.__version__}, python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
+def _host_stale() -> bool:
+    src, header = CSRC / "host.cpp", PKG.parent / "include" / "nf4b200.h"
+    if not HOST.exists() or HOST.stat().st_mtime < max(src.stat().st_mtime, header.stat().st_mtime):
+        return True
+    return f"built for {host_target()};".encode() not in HOST.read_bytes()
+
+
 def build_host(force: bool = False) -> Path:
     """The extension module, against the headers and libraries of the torch that is installed."""
-    src, header = CSRC / "host.cpp", PKG.parent / "include" / "nf4b200.h"
-    if not force and HOST.exists() and HOST.stat().st_mtime >= max(src.stat().st_mtime, header.stat().st_mtime):
+    if not force and not _host_stale():
         return HOST
     import torch
 
+    src = CSRC / "host.cpp"
     base = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parents[1]
     tmp = HOST.with_suffix(".so.tmp")
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", str(src), "-o", str(tmp),
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f'-DNF4B200_HOST_TARGET="{host_target()}"',
            f"-I{base}/include", f"-I{base}/include/torch/csrc/api/include",
            f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
            f"-L{base}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",

@@ -342,7 +342,14 @@ std::tuple<Tensor, Tensor, Tensor> rotate_bwd(const Tensor& gq, const Tensor& gk
 
 }  // namespace
 
+// What the module was compiled against; the build looks for the text in the file.
+#ifndef NF4B200_HOST_TARGET
+#define NF4B200_HOST_TARGET "unknown"
+#endif
+const char BUILT_FOR[] = "built for " NF4B200_HOST_TARGET ";";
+
 PYBIND11_MODULE(_host, m) {
+    m.attr("built_for") = py::str(BUILT_FOR + sizeof "built for " - 1, sizeof NF4B200_HOST_TARGET - 1);
     py::class_<Rotation>(m, "Rotation");
     m.def("stamps", &stamps);
     // An allocation or a launch can block (cudaMalloc, a full launch queue): other Python threads go on.

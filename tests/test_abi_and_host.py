@@ -439,3 +439,27 @@ def test_rows_view_gives_aligned_rows():
     assert all(_rows_view(t, 64).data_ptr() == t.data_ptr() for t in kept)
     odd = flat[1:1 + 5 * 63].view(5, 63)
     assert _rows_view(odd, 63).data_ptr() == odd.data_ptr()
+
+
+def test_host_module_belongs_to_the_installed_torch(library, monkeypatch, tmp_path):
+    """_host.so is built again for another torch or Python, however new the file is, and a module built
+    for another one is refused by name."""
+    import hackaton_b200
+    from hackaton_b200 import _lib, build
+
+    assert not build._host_stale() and _lib.host().built_for == build.host_target()
+    copy = tmp_path / "_host.so"
+    monkeypatch.setattr(build, "HOST", copy)
+    assert build._host_stale()
+    content = (build.PKG / "_host.so").read_bytes()
+    copy.write_bytes(content)
+    assert not build._host_stale()
+    copy.write_bytes(content.replace(b"built for torch 2", b"built for torch 1"))
+    assert build._host_stale()
+    monkeypatch.setattr(_lib, "_host_module", None)
+    other = types.ModuleType("hackaton_b200._host")
+    other.built_for = "torch 1.0, python 3.1"
+    monkeypatch.setitem(sys.modules, "hackaton_b200._host", other)
+    monkeypatch.setattr(hackaton_b200, "_host", other, raising=False)
+    with pytest.raises(RuntimeError, match="torch 1.0.*hackaton_b200.build"):
+        _lib.host()
