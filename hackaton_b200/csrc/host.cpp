@@ -79,6 +79,17 @@ Tensor scratch(int64_t bytes, const at::Device& device) {
     return at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(device));
 }
 
+// What a kernel reads besides its input has to be there: a rank-16 pair of `rows` and `cols`, a bias.
+void check_pair(const Opt& a, int64_t rows, const Opt& b, int64_t cols) {
+    TORCH_CHECK(a.has_value() == b.has_value() &&
+                    (!a.has_value() || (a->numel() >= rows * RANK && b->numel() >= cols * RANK)),
+                "rank-16 pair does not reach over ", rows, " rows and ", cols, " columns");
+}
+
+void check_bias(const Opt& bias, int64_t cols) {
+    TORCH_CHECK(!bias.has_value() || bias->numel() >= cols, "bias of ", bias->numel(), " values for ", cols, " outputs");
+}
+
 Opt half(const Opt& t) {
     if (!t.has_value()) return t;
     return t->to(at::kHalf).contiguous();
@@ -90,6 +101,8 @@ Tensor linear_fwd(int64_t w, const Tensor& x, const Opt& bias, const Opt& xa, co
     if (x.numel() == 0) return output(x, q->n_rows);
     const c10::cuda::CUDAGuard guard(x.device());
     const Tensor x2 = rows_view(x, q->n_cols);
+    check_pair(xa, x2.size(0), lora_b, q->n_rows);
+    check_bias(bias, q->n_rows);
     Tensor y = output(x, q->n_rows);
     const Opt b = half(bias);
     check(nf4b200_linear_fwd(q, x2.const_data_ptr(), x2.size(0), x2.stride(0), ptr(b), ptr(xa), ptr(lora_b),
@@ -102,6 +115,7 @@ Tensor linear_bwd_dx(int64_t w, const Tensor& dy, const Opt& u, const Opt& lora_
     if (dy.numel() == 0) return output(dy, q->n_cols);
     const c10::cuda::CUDAGuard guard(dy.device());
     const Tensor g2 = rows_view(dy, q->n_rows);
+    check_pair(u, g2.size(0), lora_a, q->n_cols);
     Tensor dx = output(dy, q->n_cols);
     check(nf4b200_linear_bwd_dx(q, g2.const_data_ptr(), g2.size(0), g2.stride(0), ptr(u), ptr(lora_a), dx.data_ptr(),
                                 q->n_cols, raw(ws), (size_t)ws_bytes, stream_of(dy)));
@@ -124,6 +138,8 @@ std::vector<Tensor> linear_fwd_group(const std::vector<int64_t>& ws_addr, const 
     const Tensor x2 = rows_view(x, weight(ws_addr[0])->n_cols);
     for (int i = 0; i < n; ++i) {
         q[i] = weight(ws_addr[i]);
+        check_pair(xas[i], x2.size(0), lora_bs[i], q[i]->n_rows);
+        check_bias(biases[i], q[i]->n_rows);
         keep.push_back(half(biases[i]));
         b[i] = ptr(keep.back());
         a[i] = ptr(xas[i]);
@@ -151,6 +167,8 @@ Tensor linear_bwd_dx_group(const std::vector<int64_t>& ws_addr, const std::vecto
         keep.push_back(rows_view(grads[i], q[i]->n_rows));
         g[i] = keep.back().const_data_ptr();
         ld[i] = keep.back().stride(0);
+        TORCH_CHECK(keep.back().size(0) == keep[0].size(0), "gradients differ in their number of rows");
+        check_pair(us[i], keep[0].size(0), lora_as[i], q[i]->n_cols);
         u[i] = ptr(us[i]);
         a[i] = ptr(lora_as[i]);
     }

@@ -100,6 +100,9 @@ def lora_side(inputs, ps, scalings, bs=None, transpose=False, zero=None):
     row count) and fp16 copies of p. With `bs` ([N, 16] each) also their fp16 copies and, with
     `transpose`, fp16 [16, N] transposes. `zero`: an fp32 buffer (a multiple of 4 elements) to fill with zeros.
     Returns (products, p16s, b16s, b16ts)."""
+    for t in inputs:     # (before anything is launched: the kernel reads two bytes per element)
+        if t.dtype != torch.float16:
+            raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {t.dtype}")
     return _lib.host().lora_side(inputs, ps, scalings, [] if bs is None else bs, transpose, zero)
 
 
@@ -129,6 +132,8 @@ class NF4LoRALinear(torch.autograd.Function):
     def forward(ctx, x, x_lora, packed, bias, state, lora_a, lora_b, scaling):
         same = x_lora is x or (x_lora.data_ptr() == x.data_ptr() and x_lora.shape == x.shape
                                and x_lora.stride() == x.stride())
+        if x_lora.numel() != x.numel():
+            raise ValueError(f"hackaton_b200: LoRA input {tuple(x_lora.shape)} for an input {tuple(x.shape)}")
         # scaling * x_l . Aᵀ [M, 16], fp16 A and B, and Bᵀ for the gradient's product
         (xa,), (a16,), (b16,), (b16t,) = lora_side([x_lora], [lora_a], [scaling], [lora_b],
                                                    transpose=any(ctx.needs_input_grad))

@@ -463,3 +463,27 @@ def test_host_module_belongs_to_the_installed_torch(library, monkeypatch, tmp_pa
     monkeypatch.setattr(hackaton_b200, "_host", other, raising=False)
     with pytest.raises(RuntimeError, match="torch 1.0.*hackaton_b200.build"):
         _lib.host()
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int8, torch.float32, torch.bfloat16])
+def test_lora_inputs_of_other_types_are_refused_before_the_launch(monkeypatch, dtype):
+    """The side kernel reads two bytes per element of its inputs; a type of one byte would be read past
+    its end. The refusal comes before anything is launched, alone and in a group."""
+    from hackaton_b200 import _lib, lora
+    from hackaton_b200.group import NF4LinearGroup, Projection
+
+    calls = []
+    host = types.SimpleNamespace(lora_side=lambda *args: calls.append(args))
+    monkeypatch.setattr(_lib, "host", lambda: host)
+    a, b = torch.zeros(16, 64), torch.zeros(32, 16)
+    x = torch.zeros(4, 64).to(dtype)
+    with pytest.raises(TypeError):
+        lora.lora_side([x], [a], [1.0], [b])
+    with pytest.raises(TypeError):
+        NF4LinearGroup.apply(x, [Projection(None, None, None, a, b)], None, a, b)
+    with pytest.raises(TypeError):
+        lora.NF4LoRALinear.apply(x, x, None, None, None, a, b, 1.0)
+    half = torch.zeros(4, 64, dtype=torch.float16)
+    with pytest.raises(ValueError):
+        lora.NF4LoRALinear.apply(half, half[:2], None, None, None, a, b, 1.0)
+    assert not calls

@@ -156,3 +156,31 @@ def test_side_products_of_ragged_inputs(cuda_lib, c, offset):
     assert float((o.double() - want).abs().max()) <= 1e-3 * float(want.abs().max())
     assert torch.equal(p16, p.half()) and torch.equal(b16, b.half()) and torch.equal(bt, b.half().t())
     assert not zero.any()
+
+
+def test_operands_that_do_not_fit_are_refused(cuda_lib):
+    """A bias, a rank-16 operand or a gradient with too few rows is refused on the host, alone and in a
+    group; the right sizes pass."""
+    from hackaton_b200.group import linear_backward_dx_group, linear_forward_group
+    from hackaton_b200.nf4 import linear_backward_dx, linear_forward
+
+    n, k, m = 128, 192, 6
+    w = synthetic_weight(n, k, True, seed=1, device="cuda")
+    x, dy = (torch.randn(m, c, device="cuda").half() for c in (k, n))
+    half = lambda *shape: torch.zeros(*shape, device="cuda", dtype=torch.float16)  # noqa: E731
+    linear_forward(x, w[0], half(n), w[1], xa=half(m, 16), lora_b=half(n, 16))
+    linear_backward_dx(dy, *w, u=half(m, 16), lora_a=half(16, k))
+    for bias, xa, b in ((half(n - 8), None, None), (None, half(m - 1, 16), half(n, 16)),
+                        (None, half(m, 16), half(n - 8, 16)), (None, half(m, 16), None)):
+        with pytest.raises(RuntimeError):
+            linear_forward(x, w[0], bias, w[1], xa=xa, lora_b=b)
+        with pytest.raises(RuntimeError):
+            linear_forward_group(x, [w], [bias], [xa], [b])
+    for u, a in ((half(m - 1, 16), half(16, k)), (half(m, 16), half(15, k)), (None, half(16, k))):
+        with pytest.raises(RuntimeError):
+            linear_backward_dx(dy, *w, u=u, lora_a=a)
+        with pytest.raises(RuntimeError):
+            linear_backward_dx_group([dy], [w], [u], [a])
+    with pytest.raises(RuntimeError):
+        linear_backward_dx_group([dy, dy[:2]], [w, w])
+    cuda_lib.device_status()
