@@ -606,6 +606,10 @@ static cudaError_t launch_gemv_x(const GemvParams& p, dim3 grid, size_t smem, cu
     if (e != cudaSuccess) return e;
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(done.load(std::memory_order_acquire) & bit)) {
+        int reserved = 0;   // the pair table's fixed address has to lie behind it
+        e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+        if (e != cudaSuccess) return e;
+        if (reserved > (int)PAIR_AT) return cudaErrorInvalidConfiguration;
         e = cudaFuncSetAttribute(nf4_gemv_kernel<NT, MT, SWIGLU, XS, WL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  XS ? GV_MAX_SMEM : GemvShape<NT, MT, SWIGLU, WL>::FIXED_BYTES + (int)PAIR_AT);
         if (e != cudaSuccess) return e;
@@ -654,7 +658,9 @@ static cudaError_t launch_gemv_t(GemvParams p, int sms, cudaStream_t stream) {
 
 template <int MT, bool SWIGLU>
 static cudaError_t launch_gemv_m(const GemvParams& p, int sms, cudaStream_t stream) {
-    if (p.m <= 8) return launch_gemv_t<1, MT, SWIGLU, 4>(p, sms, stream);
+    // (tiles of 32 rows of one weight are for more than 8 tokens)
+    if constexpr (MT == 1 || SWIGLU)
+        if (p.m <= 8) return launch_gemv_t<1, MT, SWIGLU, 4>(p, sms, stream);
     if (p.m <= 16) return launch_gemv_t<2, MT, SWIGLU, 4>(p, sms, stream);
     if (p.m <= 32) return launch_gemv_t<4, MT, SWIGLU, 4>(p, sms, stream);
     // two blocks of 32 tokens side by side: CTAs of 8 warps, two of which fit an SM
