@@ -779,6 +779,7 @@ int nf4b200_ce_stats(const void* logits, int logits_dtype, const void* targets, 
     a.entropy = static_cast<float*>(entropy); a.argmax = static_cast<long long*>(argmax);
     a.rows = rows; a.vocab = vocab; a.f32 = logits_dtype == NF4B200_F32 ? 1 : 0;
     a.status = nf4::device_status_word();
+    a.sm_count = d->sms;
     cudaError_t e = nf4::launch_ce(a, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(NF4B200_ECUDA, "ce_stats: %s", cudaGetErrorString(e));
     return NF4B200_OK;
@@ -801,6 +802,7 @@ int nf4b200_ce_grad(const void* logits, int logits_dtype, const void* targets, c
     a.scale = static_cast<const float*>(scale); a.grad = grad;
     a.rows = rows; a.vocab = vocab; a.f32 = logits_dtype == NF4B200_F32 ? 1 : 0;
     a.status = nf4::device_status_word();
+    a.sm_count = d->sms;
     cudaError_t e = nf4::launch_ce(a, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(NF4B200_ECUDA, "ce_grad: %s", cudaGetErrorString(e));
     return NF4B200_OK;

@@ -279,8 +279,8 @@ cudaError_t launch_ce(const CeArgs& a_in, cudaStream_t stream) {
     // Threads per row: small CTAs for many rows leave the shortest last wave (2048 rows: 128 threads
     // 116 us, 256: 121, 512: 127; before, with 256 threads and no loads ahead, 127), large ones give
     // few rows enough loads in flight (256 rows: 512 threads 24 us, 1024: 28).
-    if (a.rows > 8 * 148) return launch_stats<128>(a, stream);
-    if (a.rows > 4 * 148) return launch_stats<256>(a, stream);
+    if (a.rows > 8ll * a.sm_count) return launch_stats<128>(a, stream);
+    if (a.rows > 4ll * a.sm_count) return launch_stats<256>(a, stream);
     return launch_stats<512>(a, stream);
 }
 

@@ -200,6 +200,7 @@ struct CeArgs {
     int f32;
     int vec;                     // set by the launcher
     long long segments;          // set by the launcher: CTAs per row of the gradient pass
+    int sm_count;
     int* status;                 // device status word (a target beyond the vocabulary is recorded there)
 };
 cudaError_t launch_ce(const CeArgs& a, cudaStream_t stream);
