@@ -142,7 +142,10 @@ class WeightRef:
     def _order_after_build(self):
         if torch.cuda.is_current_stream_capturing():
             return   # a capture cannot wait on outside work: build the tables before capturing
-        event, stream = self._ready
+        ready = self._ready
+        if ready is None:   # (another thread has just seen the build finish)
+            return
+        event, stream = ready
         current = torch.cuda.current_stream(self.keep[0].device)
         if event.query():
             self._ready = None

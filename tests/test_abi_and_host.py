@@ -487,3 +487,13 @@ def test_lora_inputs_of_other_types_are_refused_before_the_launch(monkeypatch, d
     with pytest.raises(ValueError):
         lora.NF4LoRALinear.apply(half, half[:2], None, None, None, a, b, 1.0)
     assert not calls
+
+
+def test_scale_table_found_ready_by_another_thread(monkeypatch):
+    """Between a call's look at the pending build and its wait another thread may have seen it finish."""
+    from hackaton_b200 import nf4
+
+    ref = object.__new__(nf4.WeightRef)
+    ref.scales16, ref._ready, ref.keep = torch.zeros(1), (object(), 0), [torch.zeros(1)]
+    monkeypatch.setattr(nf4.torch.cuda, "is_current_stream_capturing", lambda: setattr(ref, "_ready", None))
+    assert ref.prepare() is ref
