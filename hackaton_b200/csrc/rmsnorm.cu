@@ -63,7 +63,9 @@ __device__ __forceinline__ void store_dx(const RmsNormArgs& a, long long idx4, f
     if (a.dx16 != nullptr) store4_any(a.dx16, idx4, 1, dx);
 }
 
-// Forward over many rows: one warp per row.
+// Forward over many rows: one warp per row. (Instances for the add ask for the mode again, although nothing
+// else comes to them: with the answer known at compile time the loads are ordered differently, and 16,384 x 3584
+// takes 110.8 us instead of 106.7.)
 template <int NV, bool ADD>
 __global__ void __launch_bounds__(RN_WARPS * 32, NV <= 16 ? 2 : 1)
 rmsnorm_rows_kernel(const RmsNormArgs a) {
@@ -76,7 +78,7 @@ rmsnorm_rows_kernel(const RmsNormArgs a) {
     float4 x[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) x[i] = __ldg(reinterpret_cast<const float4*>(a.x) + base4 + i * 32 + lane);
-    if (ADD) {
+    if (ADD && a.mode == 2) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const float4 d = load4_any(a.delta, base4 + i * 32 + lane, 1);
@@ -110,15 +112,18 @@ __device__ __forceinline__ float block_sum(float v) {
     return warp_sum(l < warps ? part[l] : 0.f);
 }
 
-// One CTA per row of hidden = 4 * h4 floats, NV float4 per thread; everything the row needs is
-// requested before the first value is used.
-template <int NV, int MODE>
-__global__ void __launch_bounds__(1024)
+// One CTA per row of hidden = 4 * h4 floats, or one warp where a CTA holds RN_WARPS narrow rows; NV float4
+// per thread; everything the row needs is requested before the first value is used.
+template <int NV, int MODE, bool WARP>
+__global__ void __launch_bounds__(WARP ? RN_WARPS * 32 : 1024)
 rmsnorm_block_kernel(const RmsNormArgs a) {
     grid_dep_wait();
     grid_dep_launch();
     const int h4 = a.hidden >> 2;
-    const long long row = blockIdx.x, base4 = row * h4;
+    const long long row = WARP ? (long long)blockIdx.x * RN_WARPS + threadIdx.y : (long long)blockIdx.x;
+    const long long base4 = row * h4;
+    if (WARP && row >= a.rows) return;
+    auto row_sum = [&](float v) { return WARP ? warp_sum(v) : block_sum(v); };
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 x[NV], w[NV], d[NV], t[NV];   // d: mode 2 the delta, modes 1 and 3 dy; t: d_total
 #pragma unroll
@@ -141,7 +146,7 @@ rmsnorm_block_kernel(const RmsNormArgs a) {
             if (MODE == 2) { x[i].x += d[i].x; x[i].y += d[i].y; x[i].z += d[i].z; x[i].w += d[i].w; }
             sum += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
         }
-        const float rstd = 1.f / sqrtf(block_sum(sum) * inv_h + a.eps);
+        const float rstd = 1.f / sqrtf(row_sum(sum) * inv_h + a.eps);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int c = threadIdx.x + i * blockDim.x;
@@ -161,7 +166,7 @@ rmsnorm_block_kernel(const RmsNormArgs a) {
         d[i].x *= w[i].x; d[i].y *= w[i].y; d[i].z *= w[i].z; d[i].w *= w[i].w;      // g
         sum += d[i].x * x[i].x + d[i].y * x[i].y + d[i].z * x[i].z + d[i].w * x[i].w;
     }
-    const float mean_gx = block_sum(sum) * inv_h;
+    const float mean_gx = row_sum(sum) * inv_h;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
@@ -173,14 +178,15 @@ rmsnorm_block_kernel(const RmsNormArgs a) {
     }
 }
 
-template <int NV>
+template <int NV, bool WARP = false>
 static cudaError_t launch_block(const RmsNormArgs& a, cudaStream_t stream) {
-    const dim3 grid((unsigned)a.rows), block((unsigned)((a.hidden / 4 + 32 * NV - 1) / (32 * NV) * 32));
+    const dim3 grid((unsigned)(WARP ? (a.rows + RN_WARPS - 1) / RN_WARPS : a.rows));
+    const dim3 block(WARP ? 32 : (unsigned)((a.hidden / 4 + 32 * NV - 1) / (32 * NV) * 32), WARP ? RN_WARPS : 1);
     switch (a.mode) {
-        case 0: return launch_pdl(rmsnorm_block_kernel<NV, 0>, grid, block, 0, stream, a);
-        case 1: return launch_pdl(rmsnorm_block_kernel<NV, 1>, grid, block, 0, stream, a);
-        case 2: return launch_pdl(rmsnorm_block_kernel<NV, 2>, grid, block, 0, stream, a);
-        default: return launch_pdl(rmsnorm_block_kernel<NV, 3>, grid, block, 0, stream, a);
+        case 0: return launch_pdl(rmsnorm_block_kernel<NV, 0, WARP>, grid, block, 0, stream, a);
+        case 1: return launch_pdl(rmsnorm_block_kernel<NV, 1, WARP>, grid, block, 0, stream, a);
+        case 2: return launch_pdl(rmsnorm_block_kernel<NV, 2, WARP>, grid, block, 0, stream, a);
+        default: return launch_pdl(rmsnorm_block_kernel<NV, 3, WARP>, grid, block, 0, stream, a);
     }
 }
 
@@ -250,6 +256,20 @@ cudaError_t launch_rmsnorm(const RmsNormArgs& a, cudaStream_t stream) {
     if (!few && !backward && a.hidden == 28 * 128)
         return a.mode == 2 ? launch_pdl(rmsnorm_rows_kernel<28, true>, grid, block, 0, stream, a)
                            : launch_pdl(rmsnorm_rows_kernel<28, false>, grid, block, 0, stream, a);
+    // Narrow rows, a warp each. A CTA of its own costs a row more than its bytes: 16,384 rows of 64 / 256 / 512
+    // take 17.7 / 18.6 / 19.1 us forward whatever the width (modes 1 to 3 the same), with a warp each 3.6 / 5.3 /
+    // 9.3 (the generic kernel: 5.7 / 8.5 / 14.9). Up to 2048 rows a CTA's shorter chain is ahead from 192 on (2048 x
+    // 256: 2.5 against 2.7 with the add); with four arrays in flight 384 needs more rows (4096: 5.1 against 6.0,
+    // 16,384: 19.0 against 15.3) and 512 never pays (19.9 against 22.4); with one up to 1024 do (16,384 x 640 19.7
+    // against 13.2, x 1024 21.4 against 18.2).
+    if (h4 <= 32) return launch_block<1, true>(a, stream);
+    if (a.rows > 2048) {
+        if (h4 <= 64) return launch_block<2, true>(a, stream);
+        if (h4 <= 128 && a.mode != 3) return launch_block<4, true>(a, stream);
+        if (h4 <= 96 && a.rows > 8192) return launch_block<4, true>(a, stream);
+        if (h4 <= 256 && a.mode == 0)
+            return launch_pdl(rmsnorm_block_kernel<8, 0, true>, grid, dim3(32, RN_WARPS), 0, stream, a);
+    }
     // float4 per thread: one where latency counts or four arrays are in flight, otherwise two
     if (h4 <= 1024 && (few || a.mode == 3 || h4 <= 128)) return launch_block<1>(a, stream);
     if (h4 <= 2048 && (few || backward || h4 <= 256)) return launch_block<2>(a, stream);

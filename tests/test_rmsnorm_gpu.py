@@ -117,7 +117,7 @@ def test_empty_and_errors(cuda_lib):
 @pytest.mark.parametrize("rows", [1, 512, 513])                     # one CTA per row up to 512 rows
 @pytest.mark.parametrize("hidden", [4, 132, 640, 1536, 3192, 3584, 4100, 8196, 16388])
 def test_widths_and_row_counts(cuda_lib, rows, hidden):
-    """Every kernel the launcher picks (row per warp, row per CTA with 1, 2, 4, 8 loads per thread,
+    """Every kernel the launcher picks (row per warp, row per CTA with 1, 2, 4 loads per thread,
     walked twice beyond 16,384), all four modes, against 64-bit arithmetic. fp32 bound: a sum of
     `hidden` squares in any order is off by at most hidden * 2^-24 relative; in practice far less.
     fp16 outputs: one rounding (2^-11)."""
@@ -146,3 +146,10 @@ def test_widths_and_row_counts(cuda_lib, rows, hidden):
         got = launch_backward(x, weight, rstd, dy, d_total, dx16)
         close(got, dx + d_total.double(), 2e-5)
         assert torch.equal(dx16, got.half())
+
+
+@pytest.mark.parametrize("rows", [2048, 2049, 8192, 8193])          # a warp per row beyond 2048, or 8192
+@pytest.mark.parametrize("hidden", [4, 124, 128, 132, 256, 260, 384, 388, 512, 516, 1024, 1028])
+def test_narrow_rows(cuda_lib, rows, hidden):
+    """Several rows per CTA: both sides of each limit of width and row count, all four modes."""
+    test_widths_and_row_counts(cuda_lib, rows, hidden)
