@@ -20,7 +20,6 @@ namespace nf4 {
 
 constexpr int CE_THREADS = 256;        // gradient
 constexpr int CE_GRAD_VECS = 4;         // 8-logit vectors per thread of the gradient
-constexpr int CE_STATS_VECS = 4;        // ... requested ahead by the statistics
 constexpr float CE_NEG = -1.0e30f;  // finite "minus infinity", as in the reference (kernels.py:36)
 
 // Running statistics of the logits seen so far, kept in the base-2 domain so that a logit costs
@@ -86,7 +85,8 @@ __device__ __forceinline__ float ce_load1(const void* row, long long i) {
     return F32 ? static_cast<const float*>(row)[i] : __half2float(static_cast<const __half*>(row)[i]);
 }
 
-template <bool F32, int THREADS>
+// VECS: 8-logit vectors that a thread requests ahead
+template <bool F32, int THREADS, int VECS>
 __global__ void __launch_bounds__(THREADS)
 ce_stats_kernel(const CeArgs a) {
     grid_dep_wait();
@@ -125,25 +125,25 @@ ce_stats_kernel(const CeArgs a) {
             st.d = fmaf(w, t, st.d);
         }
     };
-    // the next CE_STATS_VECS vectors are on their way while these are taken in
-    CeRaw<F32> next[CE_STATS_VECS];
+    // the next VECS vectors are on their way while these are taken in
+    CeRaw<F32> next[VECS];
     long long v = threadIdx.x;
     const auto fetch = [&](long long v0) {
 #pragma unroll
-        for (int u = 0; u < CE_STATS_VECS; ++u)
+        for (int u = 0; u < VECS; ++u)
             if (v0 + u * THREADS < n8) next[u].load(base, (v0 + u * THREADS) * 8);
     };
     fetch(v);
-    for (; v + (CE_STATS_VECS - 1) * THREADS < n8; v += CE_STATS_VECS * THREADS) {
-        CeRaw<F32> now[CE_STATS_VECS];
+    for (; v + (VECS - 1) * THREADS < n8; v += VECS * THREADS) {
+        CeRaw<F32> now[VECS];
 #pragma unroll
-        for (int u = 0; u < CE_STATS_VECS; ++u) now[u] = next[u];
-        fetch(v + CE_STATS_VECS * THREADS);
+        for (int u = 0; u < VECS; ++u) now[u] = next[u];
+        fetch(v + VECS * THREADS);
 #pragma unroll
-        for (int u = 0; u < CE_STATS_VECS; ++u) take(now[u], v + u * THREADS);
+        for (int u = 0; u < VECS; ++u) take(now[u], v + u * THREADS);
     }
 #pragma unroll
-    for (int u = 0; u < CE_STATS_VECS; ++u)
+    for (int u = 0; u < VECS; ++u)
         if (v + u * THREADS < n8) take(next[u], v + u * THREADS);
     for (long long i = n8 * 8 + threadIdx.x; i < a.vocab; i += THREADS) {
         const float x = ce_load1<F32>(base, i);
@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(const CeArgs a) {
     grid_dep_wait();
     grid_dep_launch();
-    const long long row = blockIdx.x / a.segments, segment = blockIdx.x % a.segments;
+    const unsigned segments = (unsigned)a.segments, row_u = blockIdx.x / segments;   // (32 bits: short CTAs)
+    const long long row = row_u, segment = blockIdx.x - row_u * segments;
     const void* base = F32 ? static_cast<const void*>(static_cast<const float*>(a.logits) + row * a.vocab)
                            : static_cast<const void*>(static_cast<const __half*>(a.logits) + row * a.vocab);
     void* out = F32 ? static_cast<void*>(static_cast<float*>(a.grad) + row * a.vocab)
@@ -254,11 +255,9 @@ ce_grad_kernel(const CeArgs a) {
     }
 }
 
-template <int THREADS>
+template <bool F32, int THREADS, int VECS>
 static cudaError_t launch_stats(const CeArgs& a, cudaStream_t stream) {
-    const dim3 grid((unsigned)a.rows), block(THREADS);
-    return a.f32 ? launch_pdl(ce_stats_kernel<true, THREADS>, grid, block, 0, stream, a)
-                 : launch_pdl(ce_stats_kernel<false, THREADS>, grid, block, 0, stream, a);
+    return launch_pdl(ce_stats_kernel<F32, THREADS, VECS>, dim3((unsigned)a.rows), dim3(THREADS), 0, stream, a);
 }
 
 cudaError_t launch_ce(const CeArgs& a_in, cudaStream_t stream) {
@@ -276,12 +275,32 @@ cudaError_t launch_ce(const CeArgs& a_in, cudaStream_t stream) {
         return a.f32 ? launch_pdl(ce_grad_kernel<true>, grid, block, 0, stream, a)
                      : launch_pdl(ce_grad_kernel<false>, grid, block, 0, stream, a);
     }
-    // Threads per row: small CTAs for many rows leave the shortest last wave (2048 rows: 128 threads
-    // 116 us, 256: 121, 512: 127; before, with 256 threads and no loads ahead, 127), large ones give
-    // few rows enough loads in flight (256 rows: 512 threads 24 us, 1024: 28).
-    if (a.rows > 8ll * a.sm_count) return launch_stats<128>(a, stream);
-    if (a.rows > 4ll * a.sm_count) return launch_stats<256>(a, stream);
-    return launch_stats<512>(a, stream);
+    // Threads per row and vectors ahead. Few rows of many logits need both for enough loads in flight; many
+    // rows need registers left for many CTAs and a short last wave, rows of few logits threads that get more
+    // than a few vectors each. us, the variants in the order of the lines below, the taken one marked *,
+    // last 256 threads without loads ahead:
+    //   fp16 64 x 151,936 12.1* 15.8 27.0, 45.2    512 x 151,936 40.8* 39.7 41.1, 52.4
+    //        1024 x 151,936 67.6 63.3* 66.9, 69.4  2048 x 151,936 127 115 112*, 123
+    //        100 x 32,000 5.8 5.8* 7.9, 11.0       600 x 32,000 17.4 14.5 13.8*, 18.4
+    //   fp32 64 x 151,936 13.5* 17.2 28.1 50.6, 49.1   256 x 151,936 32.2 29.8* 35.8 56.2, 54.2
+    //        512 x 151,936 60.6 54.1 52.9* 64.5, 62.9  2048 x 151,936 (128 threads, four ahead) 180*, 205
+    // Rows without 16-byte accesses are walked logit by logit (512 x 151,935: 256 threads 66 us, 128 102; 16,384 x
+    // 100: 35 and 21).
+    const long long sms = a.sm_count;
+    const bool wide = a.vocab >= 65536;
+    if (!a.vec && a.vocab < 8192)
+        return a.f32 ? launch_stats<true, 128, 1>(a, stream) : launch_stats<false, 128, 1>(a, stream);
+    if (!a.vec) return a.f32 ? launch_stats<true, 256, 1>(a, stream) : launch_stats<false, 256, 1>(a, stream);
+    if (a.f32) {
+        if (a.rows <= sms) return launch_stats<true, 512, 4>(a, stream);
+        if (a.rows <= 2 * sms) return launch_stats<true, 512, 2>(a, stream);
+        if (a.rows <= 4 * sms) return launch_stats<true, 256, 2>(a, stream);
+        if (!wide || a.rows <= 8 * sms) return launch_stats<true, 128, 2>(a, stream);
+        return launch_stats<true, 128, 4>(a, stream);
+    }
+    if (wide && a.rows <= 4 * sms) return launch_stats<false, 512, 4>(a, stream);
+    if (a.rows <= (wide ? 8 : 2) * sms) return launch_stats<false, 256, 4>(a, stream);
+    return launch_stats<false, 128, 4>(a, stream);
 }
 
 }  // namespace nf4

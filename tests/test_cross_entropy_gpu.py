@@ -122,15 +122,24 @@ def test_thread_counts_and_segments(cuda_lib, rows, vocab, dtype):
     close(out[0][valid], want[valid], 1e-5)
     close(out[1], torch.where(valid, -picked, 0.0), 2e-5)
     close(out[2], -(logp.exp() * logp).sum(-1), 1e-4)
-    assert torch.equal(out[3], logits.argmax(-1)) or torch.equal(
-        logits.gather(1, out[3][:, None])[:, 0], logits.amax(-1))
+    at = torch.arange(vocab, device="cuda")          # the first of equal maxima (common in fp16)
+    assert torch.equal(out[3], torch.where(logits == logits.amax(-1, keepdim=True), at, vocab).amin(-1))
     grad = logp.exp()
     grad.scatter_add_(1, targets.clamp(min=0)[:, None], torch.full_like(grad[:, :1], -1.0))
     grad = torch.where(valid[:, None], grad * 1024, 0.0)
     ce_grad(logits, targets, out[0], torch.full((1,), 1024.0, device="cuda"), logits)
-    close(logits, grad, 1e-3 if dtype == torch.float16 else 1e-3)
+    close(logits, grad, 1e-3)
     assert not logits[~valid].any()
     cuda_lib.device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("sms,extra", [(1, 0), (1, 1), (2, 0), (2, 1), (4, 0), (4, 1), (8, 0), (8, 1)])
+@pytest.mark.parametrize("vocab", [65528, 65536, 65537, 8191])     # wide from 65,536 logits on; 16-byte rows or not
+def test_thread_counts_follow_rows_and_vocabulary(cuda_lib, vocab, sms, extra, dtype):
+    """Both sides of every line of the statistics' rule: rows against multiples of the SM count."""
+    rows = sms * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    test_thread_counts_and_segments(cuda_lib, rows, vocab, dtype)
 
 
 @pytest.mark.parametrize("rows", [2048, 2049, 2600])
