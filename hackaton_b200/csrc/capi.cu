@@ -757,6 +757,7 @@ int nf4b200_qkv_rotate(const void* q, const void* k, const void* v, void* q_out,
     a.seq = (int)seq; a.heads = heads; a.kv_heads = kv_heads; a.dim = dim;
     a.padded = padded ? 1 : 0; a.backward = backward ? 1 : 0;
     a.proj_f32 = proj_dtype == NF4B200_F32 ? 1 : 0;
+    a.sm_count = d->sms;
     cudaError_t e = nf4::launch_qkv_rotate(a, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(NF4B200_ECUDA, "qkv_rotate: %s", cudaGetErrorString(e));
     return NF4B200_OK;

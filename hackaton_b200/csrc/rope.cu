@@ -8,7 +8,7 @@
 //             packed (N, heads * D) in the projections' type
 // with y1 = x1*c1 - x2*s1, y2 = x2*c2 + x1*s2 over the two halves of a head (c1/c2, s1/s2: the two
 // halves of the cos / sin rows of the token's position).
-// A work item is four q heads, or one k and one v head, of one token; dim / 16 threads share it, each with
+// Many tokens: a work item is four q heads, or one k and one v head, of one token; dim / 16 threads share it, each with
 // 8 consecutive elements of both halves (16-byte accesses for fp16). Its threads read the token's cos / sin
 // row once for all its heads (as an item per head those rows, 1 KB of fp32 each, were more L1 traffic
 // than the heads) and request all inputs of the q heads, or three copies' gradients, before using one.
@@ -194,30 +194,153 @@ qkv_rotate_kernel(const RopeArgs a) {
     rope_store8<F32>(a.ko, xi + half, fma8(d2, c2, d1, s1, -1.f));
 }
 
+// Few tokens: an item per head (every q head, k head and v head of a token), so that the work spreads over
+// more threads and no thread's chain is longer than one head's loads and stores.
+constexpr int ROPE_SLOT_COPIES = 4;   // copies whose loads are issued together in the backward
+
+template <bool F32, bool BACKWARD>
+__global__ void __launch_bounds__(256, 4)
+qkv_rotate_slot_kernel(const RopeArgs a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    const int half = a.dim / 2;
+    const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned item = gid >> a.lps_shift, slots = (unsigned)(a.heads + 2 * a.kv_heads);
+    if (item >= (unsigned)a.tokens * slots) return;
+    // Forward: a token's slots side by side. Backward: every token's q heads first, so that a CTA holds
+    // items of one weight (k / v read all their copies).
+    const unsigned q_items = (unsigned)a.tokens * (unsigned)a.heads;
+    unsigned tok_u, slot_u;
+    if (!BACKWARD) {
+        tok_u = item / slots;
+        slot_u = item - tok_u * slots;
+    } else if (item < q_items) {
+        tok_u = item / (unsigned)a.heads;
+        slot_u = item - tok_u * (unsigned)a.heads;
+    } else {
+        const unsigned r = item - q_items, kv2 = 2u * (unsigned)a.kv_heads;
+        tok_u = r / kv2;
+        slot_u = (unsigned)a.heads + (r - tok_u * kv2);
+    }
+    const int j = (int)(gid & ((1u << a.lps_shift) - 1u)) * 8;
+    const long long tok = tok_u;
+    const int slot = (int)slot_u;
+    const int b = a.b_idx[tok], t = a.t_idx[tok];
+    const int rep = a.heads / a.kv_heads;
+    const long long head_base = a.padded ? (long long)b * a.heads * a.seq + t : tok * a.heads;
+    const long long head_step = a.padded ? a.seq : 1;
+    auto out_at = [&](int head) { return (head_base + head * head_step) * a.dim + j; };
+    auto load = [](const void* p, long long idx) {
+        Raw8<BACKWARD ? false : F32> r;
+        r.load(p, idx);
+        return r.get();
+    };
+    const long long cb = (long long)b * a.cos_stride_b + (long long)t * a.cos_stride_t;
+    F8 c1, c2, s1, s2;
+    auto load_angles = [&]() {
+        Raw8<true> r;
+        r.load(a.cos, cb + j); c1 = r.get();
+        r.load(a.cos, cb + half + j); c2 = r.get();
+        r.load(a.sin, cb + j); s1 = r.get();
+        r.load(a.sin, cb + half + j); s2 = r.get();
+    };
+    if (!BACKWARD && slot < a.heads + a.kv_heads) load_angles();
+    if (slot < a.heads) {
+        const long long xi = tok * (long long)(a.heads * a.dim) + slot * a.dim + j, yi = out_at(slot);
+        if (!BACKWARD) {
+            const F8 x1 = load(a.q, xi), x2 = load(a.q, xi + half);
+            rope_store8<false>(a.qo, yi, fma8(x1, c1, x2, s1, -1.f));
+            rope_store8<false>(a.qo, yi + half, fma8(x2, c2, x1, s2, 1.f));
+        } else {
+            const F8 d1 = load(a.q, yi), d2 = load(a.q, yi + half);
+            load_angles();
+            rope_store8<F32>(a.qo, xi, fma8(d1, c1, d2, s2, 1.f));
+            rope_store8<F32>(a.qo, xi + half, fma8(d2, c2, d1, s1, -1.f));
+        }
+        return;
+    }
+    const bool is_k = slot < a.heads + a.kv_heads;
+    const int head = slot - a.heads - (is_k ? 0 : a.kv_heads);
+    const void* src = is_k ? a.k : a.v;
+    void* dst = is_k ? a.ko : a.vo;
+    const long long xi = tok * (long long)(a.kv_heads * a.dim) + head * a.dim + j;
+    if (!BACKWARD) {
+        const F8 x1 = load(src, xi), x2 = load(src, xi + half);
+        const F8 y1 = is_k ? fma8(x1, c1, x2, s1, -1.f) : x1;
+        const F8 y2 = is_k ? fma8(x2, c2, x1, s2, 1.f) : x2;
+        for (int r = 0; r < rep; ++r) {
+            rope_store8<false>(dst, out_at(head * rep + r), y1);
+            rope_store8<false>(dst, out_at(head * rep + r) + half, y2);
+        }
+        return;
+    }
+    F8 d1, d2;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d1.v[i] = d2.v[i] = 0.f;
+    for (int r0 = 0; r0 < rep; r0 += ROPE_SLOT_COPIES) {
+        // the copies' loads go out together, the sums follow in copy order
+        Raw8<false> u[ROPE_SLOT_COPIES], w[ROPE_SLOT_COPIES];
+#pragma unroll
+        for (int r = 0; r < ROPE_SLOT_COPIES; ++r) {
+            u[r].q[0] = w[r].q[0] = make_uint4(0u, 0u, 0u, 0u);
+            if (r0 + r < rep) {
+                u[r].load(src, out_at(head * rep + r0 + r));
+                w[r].load(src, out_at(head * rep + r0 + r) + half);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < ROPE_SLOT_COPIES; ++r) {
+            if (r0 + r < rep) {
+                const F8 f = u[r].get(), g = w[r].get();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    d1.v[i] += f.v[i];
+                    d2.v[i] += g.v[i];
+                }
+            }
+        }
+    }
+    if (is_k) load_angles();
+    rope_store8<F32>(dst, xi, is_k ? fma8(d1, c1, d2, s2, 1.f) : d1);
+    rope_store8<F32>(dst, xi + half, is_k ? fma8(d2, c2, d1, s1, -1.f) : d2);
+}
+
+// Few enough tokens for an item per head? In waves of its threads (four CTAs per SM): forward up to four, two where
+// k and v are not copied; backward, where an item reads all copies in a row, one, two with fp32 gradients. us, an
+// item per head against the kernel above: forward, q / kv heads 12 / 2, fp16, 256 tokens 2.2 / 3.7, 1024 3.8 / 5.1,
+// 2048 6.0 / 7.6, 4096 10.1 / 10.2, 6000 14.6 / 13.2; 28 / 4, 512 4.1 / 5.0, 2048 11.5 / 12.4, 3000 17.8 / 15.4; 16 /
+// 16, 512 4.1 / 4.5, 1024 6.7 / 6.2. Forward and backward together 12 / 2, 64 tokens 4.7 / 6.9, 1024 8.3 / 8.9, 3000
+// 17.4 / 15.9; 28 / 4, 512 8.7 / 10.2, 3000 41.7 / 35.4; fp32 projections 12 / 2, 2048 15.0 / 15.6.
+static bool rope_few(const RopeArgs& a) {
+    const long long threads = a.tokens * (a.heads + 2 * a.kv_heads) * (a.dim / 16);
+    const int waves = a.backward ? (a.proj_f32 ? 2 : 1) : (a.heads > a.kv_heads ? 4 : 2);
+    return threads <= (long long)waves * a.sm_count * 4 * 256;
+}
+
 template <bool F32, bool BACKWARD, int CTAS>
 static cudaError_t launch_rotate(RopeArgs a, cudaStream_t stream) {
     const int lps = a.dim / 16;   // threads per work item: 8 elements of each half
     a.lps_shift = 0;
     while ((1 << a.lps_shift) < lps) ++a.lps_shift;
+    const long long slots = a.tokens * (a.heads + 2 * a.kv_heads) * lps;
+    // (the limit of the 32-bit indices with an item per head)
+    if ((1 << a.lps_shift) != lps || slots >= (1ll << 31)) return cudaErrorInvalidValue;
+    if (rope_few(a))
+        return launch_pdl(qkv_rotate_slot_kernel<F32, BACKWARD>, dim3((unsigned)((slots + 255) / 256)), dim3(256), 0,
+                          stream, a);
     const long long threads =
         a.tokens * ((a.heads + ROPE_Q_HEADS - 1) / ROPE_Q_HEADS + a.kv_heads) * lps;
-    // (the limit of the 32-bit indices with an item per head)
-    if ((1 << a.lps_shift) != lps || a.tokens * (a.heads + 2 * a.kv_heads) * lps >= (1ll << 31))
-        return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)((threads + 255) / 256)), block(256);
-    return launch_pdl(qkv_rotate_kernel<F32, BACKWARD, CTAS>, grid, block, 0, stream, a);
+    return launch_pdl(qkv_rotate_kernel<F32, BACKWARD, CTAS>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,
+                      stream, a);
 }
 
 cudaError_t launch_qkv_rotate(const RopeArgs& a, cudaStream_t stream) {
     if (a.tokens <= 0) return cudaSuccess;
     // Three CTAs per SM (80 registers, a few spilled) keep the most loads in flight; two (no spills) are
-    // better where the launch is short or a forward item holds fp32 loads (us, three against two: 16,384
-    // tokens 36.7 / 40.0, 2048 tokens 7.3 / 6.5, 8192 tokens of fp32 projections 28.6 / 24.8).
+    // better where a forward item holds fp32 loads (8192 tokens of fp32 projections 25.3 us against 29.5).
     if (a.backward)
         return a.proj_f32 ? launch_rotate<true, true, 3>(a, stream) : launch_rotate<false, true, 3>(a, stream);
-    if (a.proj_f32) return launch_rotate<true, false, 2>(a, stream);
-    return a.tokens * a.heads >= 4096ll * 12 ? launch_rotate<false, false, 3>(a, stream)
-                                             : launch_rotate<false, false, 2>(a, stream);
+    return a.proj_f32 ? launch_rotate<true, false, 2>(a, stream) : launch_rotate<false, false, 3>(a, stream);
 }
 
 }  // namespace nf4

@@ -177,3 +177,14 @@ def test_heads_not_in_fours_and_copies_not_in_threes(cuda_lib, heads, kv_heads, 
     tol = dict(rtol=2.0 ** -10, atol=2e-3) if dtype == torch.float16 else dict(rtol=1e-5, atol=2e-5)
     for o, w in zip(got, (back(gq), back(gk), gv.reshape(tokens, -1))):
         torch.testing.assert_close(o.double(), w, **tol)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(12, 2, 128), (5, 1, 64), (6, 6, 256)])
+@pytest.mark.parametrize("waves", [1, 2, 4])
+@pytest.mark.parametrize("extra", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_both_sides_of_the_item_rule(cuda_lib, heads, kv_heads, dim, waves, extra, dtype):
+    """The largest token count that takes an item per head, and the next one, in each direction."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tokens = waves * sms * 1024 // ((heads + 2 * kv_heads) * (dim // 16)) + extra
+    test_heads_not_in_fours_and_copies_not_in_threes(cuda_lib, heads, kv_heads, dim, tokens, dtype)
