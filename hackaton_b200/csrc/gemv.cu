@@ -117,10 +117,14 @@ __device__ __forceinline__ void mma_16816_first(float (&d)[4], uint32_t a0, uint
 // has no static shared memory, so its dynamic part starts right there).
 constexpr uint32_t PAIR_AT = 2048;
 
+// The table is written again when a CTA walks on to another member, so the compiler has to know that a look-up
+// reads memory. IN_ORDER: volatile, which also keeps the look-ups in program order; an ordinary load may be moved
+// between the barriers. A decode step of the 3584-wide network at 16 tokens (4 layers) takes 519 us in order and
+// 534 with ordinary loads, one of the 1536-wide network at 32 tokens (10 layers) 529 and 518.
+template <bool IN_ORDER>
 __device__ __forceinline__ uint32_t pair_lookup(uint32_t offset) {
+    if (!IN_ORDER) return *static_cast<const uint32_t*>(__cvta_shared_to_generic(offset + PAIR_AT));
     uint32_t v;
-    // (volatile: the table is written again when a CTA walks on to another member, so a value is only good
-    // on this side of the barriers around that)
     asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(offset), "n"(PAIR_AT));
     return v;
 }
@@ -228,8 +232,8 @@ nf4_gemv_kernel(const __grid_constant__ GemvParams p) {
     auto pairs = [&](int mt, uint32_t w, uint32_t (&o)[8], int at) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            o[at + i] = pair_lookup(SWIGLU ? __byte_perm(w, lane4 + mt * 128, 0x7604u + (i << 4))
-                                           : __byte_perm(w, 0u, 0x4440u + i) * 128u + lane4);
+            o[at + i] = pair_lookup<NT <= 2>(SWIGLU ? __byte_perm(w, lane4 + mt * 128, 0x7604u + (i << 4))
+                                                    : __byte_perm(w, 0u, 0x4440u + i) * 128u + lane4);
     };
     const uint32_t ring = PAIR_AT + Shape::TABLE_BYTES + warp * Shape::RING;   // shared-memory address
     const uint8_t* const ring_ptr = table + Shape::TABLE_BYTES + warp * Shape::RING;
@@ -656,15 +660,20 @@ static cudaError_t launch_gemv_t(GemvParams p, int sms, cudaStream_t stream) {
     return launch_gemv_x<NT, MT, SWIGLU, false, WL>(p, grid, fixed, stream);
 }
 
-template <int MT, bool SWIGLU>
+// CTAs of 2^WL warps; token blocks of 8, as many as there are up to four.
+template <int MT, bool SWIGLU, int WL>
 static cudaError_t launch_gemv_m(const GemvParams& p, int sms, cudaStream_t stream) {
-    // (tiles of 32 rows of one weight are for more than 8 tokens)
-    if constexpr (MT == 1 || SWIGLU)
-        if (p.m <= 8) return launch_gemv_t<1, MT, SWIGLU, 4>(p, sms, stream);
-    if (p.m <= 16) return launch_gemv_t<2, MT, SWIGLU, 4>(p, sms, stream);
-    if (p.m <= 32) return launch_gemv_t<4, MT, SWIGLU, 4>(p, sms, stream);
-    // two blocks of 32 tokens side by side: CTAs of 8 warps, two of which fit an SM
-    if constexpr (MT == 1 && !SWIGLU) return launch_gemv_t<4, 1, false, 3>(p, sms, stream);
+    constexpr bool PAIRED = MT == 2;   // (tiles of 32 rows: not all token blocks, see launch_gemv_group)
+    if constexpr (!PAIRED || SWIGLU)
+        if (p.m <= 8) return launch_gemv_t<1, MT, SWIGLU, WL>(p, sms, stream);
+    if (p.m <= 16) return launch_gemv_t<2, MT, SWIGLU, WL>(p, sms, stream);
+    if constexpr (!PAIRED)
+        if (p.m <= 24) return launch_gemv_t<3, MT, SWIGLU, WL>(p, sms, stream);
+    if (p.m <= 32) return launch_gemv_t<4, MT, SWIGLU, WL>(p, sms, stream);
+    // two blocks of tokens side by side: CTAs of 8 warps, two of which fit an SM
+    if constexpr (!PAIRED && WL == 3)
+        return p.m <= 48 ? launch_gemv_t<3, MT, SWIGLU, WL>(p, sms, stream)
+                         : launch_gemv_t<4, MT, SWIGLU, WL>(p, sms, stream);
     return cudaErrorInvalidValue;
 }
 
@@ -687,18 +696,31 @@ static GemvParams gemv_forward_params(const GemmGroupArgs& ga, int rows) {
 cudaError_t launch_gemv_group(const GemmGroupArgs& ga, cudaStream_t stream) {
     const GemmArgs& a = ga.item[0];
     const int sms = a.sm_count > 0 ? a.sm_count : 148;
-    // Tiles of 32 rows read the activations half as often: they pay with more than 8 tokens where they
-    // still occupy most SMs (us at 16 tokens, 32 against 16 rows: down_proj 3584 x 18944 21.7 against
-    // 26.9, 1536 x 8960 12.2 against 8.6).
     long long rows = 0;
-    bool wide = a.m > 8 && a.m <= 32;
+    bool wide = a.m > 8 && (a.m <= 16 || a.m > 24 || a.k_w >= 8192) && a.m <= 32;
     for (int i = 0; i < ga.count; ++i) {
         wide = wide && ga.item[i].n_w % 32 == 0;
         rows += ga.item[i].n_w;
     }
-    if (rows / 32 * 4 < 3ll * sms) wide = false;
-    if (wide) return launch_gemv_m<2, false>(gemv_forward_params(ga, 2 * GV_ROWS), sms, stream);
-    return launch_gemv_m<1, false>(gemv_forward_params(ga, GV_ROWS), sms, stream);
+    const bool small = rows * a.k_w <= (1ll << 22), one_tile = rows <= (long long)GV_ROWS * sms;
+    // Tiles of 32 rows read the activations half as often: they pay with more than 8 tokens where they
+    // still occupy most SMs and a warp's slice of K is long (us, 32 against 16 rows: at 16 tokens 3584 x 18944
+    // 21.9 against 27.0, 8960 x 1536 6.4 against 7.0, 1536 x 8960 12.2 against 8.6; at 32 tokens 4096 x 4096 10.9
+    // against 11.6, 4096 x 1024 6.0 against 5.3). 17 to 24 tokens leave a fourth token block of them idle: 3584 x
+    // 3584 at 24 tokens 10.0 against 8.9 with three, 3584 x 18944 30.5 against 31.8.
+    if (wide && !small && rows / 32 * 4 >= 3ll * sms)
+        return launch_gemv_m<2, false, 4>(gemv_forward_params(ga, 2 * GV_ROWS), sms, stream);
+    const GemvParams p = gemv_forward_params(ga, GV_ROWS);
+    // Small weights: a CTA's 32 KB pair table and the fold over its warps weigh more than the contraction, so
+    // smaller CTAs, spread over more SMs (us, CTAs of 16 / 8 / 4 warps): 256 x 256, 8 tokens 2.9 / 1.9 / 1.7, 16
+    // tokens 3.0 / 2.3 / 2.0; 512 x 512, 8 tokens 2.4 / 2.0 / 2.1, 32 tokens 3.9 / 2.9 / 3.0; 1024 x 1024, 8 tokens
+    // 2.5 / 2.4 / 2.6, 32 tokens 3.8 / 3.6 / 3.7. Larger ones stay with 16 warps: by itself 1536 x 1536 at 16 tokens
+    // takes 3.7 / 3.3 / 3.7, but two CTAs per SM leave the next kernel of a stream no room to set itself up, and a
+    // decode step of the 1536-wide network got 2 % slower (4 % at 32 tokens).
+    // More than 32 tokens, in two blocks: 1536 x 1536 at 40 tokens 5.4 with three token blocks each, 6.1 with four.
+    if (a.m <= 32 && one_tile && p.k_w <= 4 * 64) return launch_gemv_m<1, false, 2>(p, sms, stream);
+    if (a.m > 32 || (one_tile && p.k_w <= 16 * 64)) return launch_gemv_m<1, false, 3>(p, sms, stream);
+    return launch_gemv_m<1, false, 4>(p, sms, stream);
 }
 
 bool gemv_swiglu_eligible(const GemmGroupArgs& ga) {
@@ -713,7 +735,7 @@ cudaError_t launch_gemv_swiglu(const GemmGroupArgs& ga, __half* hidden, cudaStre
     const int sms = ga.item[0].sm_count > 0 ? ga.item[0].sm_count : 148;
     GemvParams p = gemv_forward_params(ga, GV_ROWS);
     p.hidden = hidden;
-    return launch_gemv_m<2, true>(p, sms, stream);
+    return launch_gemv_m<2, true, 4>(p, sms, stream);
 }
 
 // Row slabs of the streaming backward: enough CTAs (k-blocks x slabs) for about three per SM, slabs

@@ -227,6 +227,26 @@ def test_streaming_forward_every_plan(cuda_lib, m, k):
     assert cuda_lib.device_status() == 0
 
 
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49])    # edges of one to four token blocks
+@pytest.mark.parametrize("k,groups", [
+    (64, ((16,), (64, 16))), (256, ((256,), (2368,), (2384,))), (320, ((2368,), (2384,))),
+    (1536, ((2304, 64), (2304, 80))), (1600, ((272,),)), (1024, ((4096,), (4112,))), (8192, ((3552,),))])
+def test_streaming_forward_cta_sizes(cuda_lib, m, k, groups):
+    """Both sides of the rules for CTAs of 4, 8 and 16 warps and for tiles of 32 rows (k-blocks, one tile
+    per SM, 2^22 weights, token blocks), against the fp32 product of the standalone decode."""
+    from hackaton_b200.group import linear_forward_group
+    from hackaton_b200.nf4 import dequantize_nf4
+
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(m + k), device="cuda").half()
+    for group in groups:
+        weights = [synthetic_weight(n, k, True, seed=n, device="cuda") for n in group]
+        weights = [(p, _odd_tables(s, i)) if i else (p, s) for i, (p, s) in enumerate(weights)]
+        for y, (p, s) in zip(linear_forward_group(x, weights), weights):
+            want = x.float() @ dequantize_nf4(p, s).float().t()
+            assert float((y.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+    assert cuda_lib.device_status() == 0
+
+
 def test_streaming_forward_many_row_tiles(cuda_lib):
     """More tiles than two rounds of every SM (the CTAs walk several sets), rows strided and tokens
     past the last one never written."""
