@@ -35,8 +35,6 @@ void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.devic
 
 const void* ptr(const Opt& t) { return t.has_value() ? t->const_data_ptr() : nullptr; }
 
-void* raw(const Opt& t) { return t.has_value() ? t->data_ptr() : nullptr; }
-
 const nf4b200_weight* weight(int64_t address) { return reinterpret_cast<const nf4b200_weight*>(address); }
 
 // Where the tensors of a weight lie and how often each has been written (inference tensors do not count
@@ -74,10 +72,15 @@ Tensor output(const Tensor& like, int64_t cols, at::ScalarType type = at::kHalf)
     return at::empty(shape, like.options().dtype(type).memory_format(c10::nullopt));
 }
 
-// Scratch of one call on the current stream.
-Tensor scratch(int64_t bytes, const at::Device& device) {
-    return at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(device));
-}
+// Scratch of one call on the current stream (see hackaton_b200.nf4.scratch_bytes): the allocator hands it
+// out again only behind the work of that stream.
+struct Scratch {
+    Tensor buffer;
+    Scratch(int64_t bytes, const Tensor& like) {
+        if (bytes > 0) buffer = at::empty({bytes}, like.options().dtype(at::kByte).memory_format(c10::nullopt));
+    }
+    void* get() const { return buffer.defined() ? buffer.data_ptr() : nullptr; }
+};
 
 // What a kernel reads besides its input has to be there: a rank-16 pair of `rows` and `cols`, a bias.
 void check_pair(const Opt& a, int64_t rows, const Opt& b, int64_t cols) {
@@ -95,8 +98,7 @@ Opt half(const Opt& t) {
     return t->to(at::kHalf).contiguous();
 }
 
-Tensor linear_fwd(int64_t w, const Tensor& x, const Opt& bias, const Opt& xa, const Opt& lora_b, const Opt& ws,
-                  int64_t ws_bytes) {
+Tensor linear_fwd(int64_t w, const Tensor& x, const Opt& bias, const Opt& xa, const Opt& lora_b, int64_t ws_bytes) {
     const nf4b200_weight* q = weight(w);
     if (x.numel() == 0) return output(x, q->n_rows);
     const c10::cuda::CUDAGuard guard(x.device());
@@ -105,25 +107,27 @@ Tensor linear_fwd(int64_t w, const Tensor& x, const Opt& bias, const Opt& xa, co
     check_bias(bias, q->n_rows);
     Tensor y = output(x, q->n_rows);
     const Opt b = half(bias);
+    const Scratch ws(ws_bytes, x);
     check(nf4b200_linear_fwd(q, x2.const_data_ptr(), x2.size(0), x2.stride(0), ptr(b), ptr(xa), ptr(lora_b),
-                             y.data_ptr(), q->n_rows, raw(ws), (size_t)ws_bytes, stream_of(x)));
+                             y.data_ptr(), q->n_rows, ws.get(), (size_t)ws_bytes, stream_of(x)));
     return y;
 }
 
-Tensor linear_bwd_dx(int64_t w, const Tensor& dy, const Opt& u, const Opt& lora_a, const Opt& ws, int64_t ws_bytes) {
+Tensor linear_bwd_dx(int64_t w, const Tensor& dy, const Opt& u, const Opt& lora_a, int64_t ws_bytes) {
     const nf4b200_weight* q = weight(w);
     if (dy.numel() == 0) return output(dy, q->n_cols);
     const c10::cuda::CUDAGuard guard(dy.device());
     const Tensor g2 = rows_view(dy, q->n_rows);
     check_pair(u, g2.size(0), lora_a, q->n_cols);
     Tensor dx = output(dy, q->n_cols);
+    const Scratch ws(ws_bytes, dy);
     check(nf4b200_linear_bwd_dx(q, g2.const_data_ptr(), g2.size(0), g2.stride(0), ptr(u), ptr(lora_a), dx.data_ptr(),
-                                q->n_cols, raw(ws), (size_t)ws_bytes, stream_of(dy)));
+                                q->n_cols, ws.get(), (size_t)ws_bytes, stream_of(dy)));
     return dx;
 }
 
 std::vector<Tensor> linear_fwd_group(const std::vector<int64_t>& ws_addr, const Tensor& x, const Opts& biases,
-                                     const Opts& xas, const Opts& lora_bs, const Opt& ws, int64_t ws_bytes) {
+                                     const Opts& xas, const Opts& lora_bs, int64_t ws_bytes) {
     const int n = (int)ws_addr.size();
     TORCH_CHECK(n >= 1 && n <= MAX_GROUP, "a group holds 1..", MAX_GROUP, " projections, got ", n);
     std::vector<Tensor> ys;
@@ -147,13 +151,14 @@ std::vector<Tensor> linear_fwd_group(const std::vector<int64_t>& ws_addr, const 
         y[i] = ys[i].data_ptr();
         ld[i] = q[i]->n_rows;
     }
+    const Scratch ws(ws_bytes, x);
     check(nf4b200_linear_fwd_group(n, q, x2.const_data_ptr(), x2.size(0), x2.stride(0), b, a, l, y, ld,
-                                   raw(ws), (size_t)ws_bytes, stream_of(x)));
+                                   ws.get(), (size_t)ws_bytes, stream_of(x)));
     return ys;
 }
 
 Tensor linear_bwd_dx_group(const std::vector<int64_t>& ws_addr, const std::vector<Tensor>& grads, const Opts& us,
-                           const Opts& lora_as, const Opt& ws, int64_t ws_bytes) {
+                           const Opts& lora_as, int64_t ws_bytes) {
     const int n = (int)ws_addr.size();
     TORCH_CHECK(n >= 1 && n <= MAX_GROUP && (int)grads.size() == n, "a group holds 1..", MAX_GROUP, " projections");
     if (grads[0].numel() == 0) return output(grads[0], weight(ws_addr[0])->n_cols);
@@ -174,8 +179,8 @@ Tensor linear_bwd_dx_group(const std::vector<int64_t>& ws_addr, const std::vecto
     }
     const int64_t m = keep[0].size(0), cols = q[0]->n_cols;
     Tensor dx = output(grads[0], cols);
-    check(nf4b200_linear_bwd_dx_group(n, q, g, m, ld, u, a, dx.data_ptr(), cols, raw(ws),
-                                      (size_t)ws_bytes, stream_of(dx)));
+    const Scratch ws(ws_bytes, dx);
+    check(nf4b200_linear_bwd_dx_group(n, q, g, m, ld, u, a, dx.data_ptr(), cols, ws.get(), (size_t)ws_bytes, stream_of(dx)));
     return dx;
 }
 
@@ -372,7 +377,6 @@ PYBIND11_MODULE(_host, m) {
     m.def("stamps", &stamps);
     // An allocation or a launch can block (cudaMalloc, a full launch queue): other Python threads go on.
     using unlocked = py::call_guard<py::gil_scoped_release>;
-    m.def("scratch", &scratch, unlocked());
     m.def("linear_fwd", &linear_fwd, unlocked());
     m.def("linear_bwd_dx", &linear_bwd_dx, unlocked());
     m.def("linear_fwd_group", &linear_fwd_group, unlocked());

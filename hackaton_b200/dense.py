@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .nf4 import _rows_view, _stream_ptr, _workspace
+from .nf4 import _rows_view, _stream_ptr, scratch
 
 
 def fp16_linear(x, weight, transposed=False, bias=None, out=None):
@@ -43,7 +43,7 @@ def fp16_linear(x, weight, transposed=False, bias=None, out=None):
         return y if out is not None else y.reshape(*x.shape[:-1], out_cols)
     if bias is not None:
         bias = bias.to(torch.float16).contiguous()
-    ws, ws_bytes = _workspace(x.device, n, k, m, bool(transposed))
+    ws, ws_bytes = scratch(x.device, "nf4b200_workspace_bytes", n, k, m, int(bool(transposed)))
     with torch.cuda.device(x.device):
         _lib.check(_lib.lib().nf4b200_fp16_linear(
             weight.data_ptr(), n, k, weight.stride(0), x2.data_ptr(), m, x2.stride(0),

@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from .lora import RANK, grad_buffer, lora_grad_batch, lora_side
-from .nf4 import _require, _rows, scratch_for, weight_ref
+from .nf4 import _require, _rows, scratch_bytes, streams, weight_ref
 
 MAX_GROUP = 4
 
@@ -38,8 +38,8 @@ class Projection:
 
 def _workspace(device, rows, cols, m, backward):
     if m == 0:
-        return None, 0
-    return scratch_for(device, "nf4b200_workspace_bytes_group", len(rows), tuple(rows), cols, m, int(backward))
+        return 0
+    return scratch_bytes(device, "nf4b200_workspace_bytes_group", len(rows), tuple(rows), cols, m, int(backward))
 
 
 def _refs(items):
@@ -65,10 +65,11 @@ def linear_forward_group(x, weights: Sequence, biases=None, xas=None, lora_bs=No
     cols = refs[0].cols
     if x.shape[-1] != cols:
         raise ValueError(f"input has {x.shape[-1]} features, weights expect {cols}")
-    ws, ws_bytes = _workspace(x.device, [r.rows for r in refs], cols, _rows(x), False)
+    m = _rows(x)
+    ws_bytes = 0 if streams(m, *refs) else _workspace(x.device, [r.rows for r in refs], cols, m, False)
     return _lib.host().linear_fwd_group(
         [r.address for r in refs], x, none if biases is None else list(biases), none if xas is None else list(xas),
-        none if lora_bs is None else list(lora_bs), ws, ws_bytes)
+        none if lora_bs is None else list(lora_bs), ws_bytes)
 
 
 def linear_backward_dx_group(grads: Sequence[torch.Tensor], weights: Sequence, us=None, lora_as=None):
@@ -80,9 +81,9 @@ def linear_backward_dx_group(grads: Sequence[torch.Tensor], weights: Sequence, u
             raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {g.dtype}")
         if g.shape[-1] != r.rows:
             raise ValueError(f"gradient has {g.shape[-1]} features, weight gives {r.rows}")
-    ws, ws_bytes = _workspace(grads[0].device, [r.rows for r in refs], refs[0].cols, _rows(grads[0]), True)
+    ws_bytes = _workspace(grads[0].device, [r.rows for r in refs], refs[0].cols, _rows(grads[0]), True)
     return _lib.host().linear_bwd_dx_group([r.address for r in refs], list(grads), none if us is None else list(us),
-                                           none if lora_as is None else list(lora_as), ws, ws_bytes)
+                                           none if lora_as is None else list(lora_as), ws_bytes)
 
 
 class NF4LinearGroup(torch.autograd.Function):

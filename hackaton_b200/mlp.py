@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from .group import Projection, _refs, linear_backward_dx_group
-from .nf4 import _rows_view, _stream_ptr, scratch_for
+from .nf4 import _rows_view, _stream_ptr, scratch
 
 
 def swiglu_forward(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
@@ -92,7 +92,7 @@ def gate_up_swiglu_forward(x, gate_w, up_w, keep: bool):
     gate = torch.empty_like(hidden) if keep else None
     up = torch.empty_like(hidden) if keep else None
     if m > 0:
-        ws, ws_bytes = scratch_for(x.device, "nf4b200_gate_up_swiglu_workspace_bytes", rows, cols, m, int(keep))
+        ws, ws_bytes = scratch(x.device, "nf4b200_gate_up_swiglu_workspace_bytes", rows, cols, m, int(keep))
         with torch.cuda.device(x.device):
             _lib.check(_lib.lib().nf4b200_gate_up_swiglu_fwd(
                 ctypes.byref(refs[0].struct), ctypes.byref(refs[1].struct), x2.data_ptr(), m,
@@ -141,7 +141,7 @@ def linear_backward_dx_swiglu(grad_out, down_w, gate, up):
     if m == 0:
         return d_gate, d_up
     device = g2.device
-    ws, ws_bytes = scratch_for(device, "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", ref.rows, ref.cols, m)
+    ws, ws_bytes = scratch(device, "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", ref.rows, ref.cols, m)
     with torch.cuda.device(device):
         _lib.check(_lib.lib().nf4b200_linear_bwd_dx_swiglu(
             ctypes.byref(ref.struct), g2.data_ptr(), m, g2.stride(0), gate.data_ptr(), up.data_ptr(),

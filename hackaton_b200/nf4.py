@@ -203,9 +203,13 @@ def _stream_ptr(device):
 _ws_need = {}      # (device, C function, its arguments) -> bytes of scratch under the SM limit in force
 
 
-def scratch_for(device, query, *sizes):
-    """(buffer, bytes) for a call on the current stream, or (None, 0). `query`: the C function that says
-    how much a call of these `sizes` (numbers, or tuples for arrays of them) takes."""
+def scratch_bytes(device, query, *sizes):
+    """What a call takes besides its operands. `query`: the C function that says how much a call of these
+    `sizes` (numbers, or tuples for arrays of them) needs. Every call takes a buffer of its own from torch's
+    allocator and drops it after the launch: the allocator hands it out again only behind the work of
+    the stream it was taken on, and a captured graph's lies in the graph's own pool for as long as the
+    graph lives. (A buffer kept per stream is neither: one that grows frees memory a captured graph still
+    writes, and two threads on a stream would interleave their launches on it.)"""
     key = (device.index, query, sizes)
     need = _ws_need.get(key)
     if need is None:
@@ -215,23 +219,26 @@ def scratch_for(device, query, *sizes):
         if need < 0:
             _lib.check(need)
         _ws_need[key] = need
-    return _scratch(device, need) if need else (None, 0)
+    return need
+
+
+def scratch(device, query, *sizes):
+    """(buffer, bytes) for one call on the current stream, uninitialised, or (None, 0)."""
+    need = scratch_bytes(device, query, *sizes)
+    return (torch.empty(need, dtype=torch.uint8, device=device), need) if need else (None, 0)
+
+
+def streams(m, *refs):
+    """Whether a forward call with `m` rows goes to the weight-streaming kernel, which takes no scratch.
+    (Only a hint: a call without scratch that lands on the tensor-core kernel is not split along K.)"""
+    return m <= 32 and all(r.scales16 is not None and r.rows % 16 == 0 for r in refs)
 
 
 def _workspace(device, n_rows, n_cols, m, backward):
-    """Split-K scratch for one GEMM call on the current stream: (buffer, bytes) or (None, 0)."""
+    """Split-K scratch of one GEMM call: (None, bytes), the buffer is the call's own business."""
     if m == 0:
         return None, 0
-    return scratch_for(device, "nf4b200_workspace_bytes", n_rows, n_cols, m, int(backward))
-
-
-def _scratch(device, need):
-    """(buffer, bytes) for one call, uninitialised. Every call takes its own from torch's allocator and
-    drops it after the launch: the allocator hands it out again only behind the work of the stream it
-    was taken on, and a captured graph's lies in the graph's own pool for as long as the graph lives.
-    (A buffer kept per stream is neither: one that grows frees memory a captured graph still writes,
-    and two threads on a stream would interleave their launches on it.)"""
-    return _lib.host().scratch(need, device), need
+    return None, scratch_bytes(device, "nf4b200_workspace_bytes", n_rows, n_cols, m, int(backward))
 
 
 def _require(packed, state):
@@ -281,8 +288,9 @@ def linear_forward(x, packed, bias, state, xa=None, lora_b=None):
         raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {x.dtype}")
     if x.shape[-1] != ref.cols:
         raise ValueError(f"input has {x.shape[-1]} features, weight expects {ref.cols}")
-    ws, ws_bytes = _workspace(x.device, ref.rows, ref.cols, _rows(x), False)
-    return _lib.host().linear_fwd(ref.address, x, bias, xa, lora_b, ws, ws_bytes)
+    m = _rows(x)
+    ws_bytes = 0 if streams(m, ref) else _workspace(x.device, ref.rows, ref.cols, m, False)[1]
+    return _lib.host().linear_fwd(ref.address, x, bias, xa, lora_b, ws_bytes)
 
 
 def linear_backward_dx(grad_output, packed, state, u=None, lora_a=None):
@@ -294,8 +302,8 @@ def linear_backward_dx(grad_output, packed, state, u=None, lora_a=None):
         raise TypeError(f"hackaton_b200: the fused NF4 linear computes in fp16, got {grad_output.dtype}")
     if grad_output.shape[-1] != ref.rows:
         raise ValueError(f"gradient has {grad_output.shape[-1]} features, weight gives {ref.rows}")
-    ws, ws_bytes = _workspace(grad_output.device, ref.rows, ref.cols, _rows(grad_output), True)
-    return _lib.host().linear_bwd_dx(ref.address, grad_output, u, lora_a, ws, ws_bytes)
+    _, ws_bytes = _workspace(grad_output.device, ref.rows, ref.cols, _rows(grad_output), True)
+    return _lib.host().linear_bwd_dx(ref.address, grad_output, u, lora_a, ws_bytes)
 
 
 class NF4Linear(torch.autograd.Function):

@@ -354,13 +354,12 @@ def test_sm_limit_drops_every_scratch_size(monkeypatch):
 
     monkeypatch.setattr(_lib, "lib", Library)
     monkeypatch.setattr(nf4, "_ws_need", {})
-    monkeypatch.setattr(nf4, "_scratch", lambda device, need: (None, need))
     monkeypatch.setattr(nf4.torch.cuda, "device", lambda d: __import__("contextlib").nullcontext())
     device = torch.device("cuda", 0)
     calls = [lambda: nf4._workspace(device, 64, 64, 4, False), lambda: nf4._workspace(device, 64, 64, 4, True),
-             lambda: group._workspace(device, [64, 64], 64, 4, False),
-             lambda: mlp.scratch_for(device, "nf4b200_gate_up_swiglu_workspace_bytes", 64, 64, 4, 1),
-             lambda: mlp.scratch_for(device, "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", 64, 64, 4)]
+             lambda: (None, group._workspace(device, [64, 64], 64, 4, False)),
+             lambda: (None, nf4.scratch_bytes(device, "nf4b200_gate_up_swiglu_workspace_bytes", 64, 64, 4, 1)),
+             lambda: (None, nf4.scratch_bytes(device, "nf4b200_linear_bwd_dx_swiglu_workspace_bytes", 64, 64, 4))]
     for _ in range(2):
         assert all(call()[1] == 256 for call in calls)
     assert len(asked) == len(calls)
