@@ -534,7 +534,7 @@ int64_t nf4b200_gate_up_swiglu_workspace_bytes(int64_t n_rows, int64_t n_cols, i
     if (n_rows <= 0 || n_cols <= 0 || m <= 0)
         return fail(NF4B200_EINVAL, "gate_up_swiglu_workspace_bytes: bad shape");
     if (m > 256) return 0;  // epilogue-fused kernel: no scratch
-    // (up to 64 rows the streaming kernel forms the product too, but only for weights that bring a
+    // (up to 32 rows the streaming kernel forms the product too, but only for weights that bring a
     // scale table: the scratch covers a call without one)
     long long rows[2] = {n_rows, n_rows};
     const nf4::GemmPlan pl = nf4::plan_gemm_group(m, rows, 2, n_cols, false, gemm_sms(d));

@@ -194,8 +194,8 @@ ce_stats_kernel(const CeArgs a) {
 // A CTA handles CE_GRAD_VECS * 8 * 256 consecutive logits of a row (and the row's last CTA the
 // remainder that is no whole vector). Short CTAs in row order leave no partly filled last wave, and
 // the logits wait in registers as they lie in memory (34 registers), so that an SM holds enough of
-// them: 2048 x 151,936 fp16 184 us = 1.03 of the copy bandwidth; one 256-thread CTA per row, 1.7
-// waves, took 235.
+// them: 2048 x 151,936 fp16 184 to 199 us from one GPU to another = 1.03 to 0.97 of the copy bandwidth; one
+// 256-thread CTA per row, 1.7 waves, took 235.
 template <bool F32>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(const CeArgs a) {

@@ -6,7 +6,7 @@
 //   3  backward + the gradient that reaches the sum directly: dx += d_total
 // x, w, s, dx, d_total fp32; y (and dy) fp32 or fp16 (the projections that follow read fp16). Modes
 // 1 and 3 also write dx in fp16 where asked: the gradient of mode 2's delta, without a second pass
-// over dx (16,384 x 1536: 54 + 22 us as a kernel and a cast, 66 as one kernel).
+// over dx (16,384 x 1536: 57 + 22 us as a kernel and a cast, 66 as one kernel).
 // HBM bound: 6 to 16 bytes per element. A row is read once into registers with 16-byte loads that
 // are all in flight together, and every output is written once. Who owns a row depends on what has
 // to be in flight (us measured, one CTA per row against one warp per row):

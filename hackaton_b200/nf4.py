@@ -60,7 +60,9 @@ def can_dequantize(packed, state):
 
 
 # Fused GEMM calls fetch ready-made fp16 block scales (built once per weight) instead of gathering
-# absmax / absmax2 on every call. Same results bit for bit; NF4B200_NO_PREPARED=1 turns it off.
+# absmax / absmax2 on every call; NF4B200_NO_PREPARED=1 turns it off. The tensor-core kernel gives the same
+# bits either way; the weight-streaming kernels (few rows) need the table and scale fp32 sums instead of
+# rounding each weight to fp16.
 PREPARED_SCALES = os.environ.get("NF4B200_NO_PREPARED", "0") != "1"
 
 
