@@ -221,40 +221,42 @@ def step_functional(layer, acts):
     their input, so each group is one launch forward and one launch (summed dX) backward, as the
     model's own data flow has it. Returns the outputs."""
     from hackaton_b200.group import linear_backward_dx_group, linear_forward_group
-    from hackaton_b200.lora import lora_down_batch, lora_grad_batch
+    from hackaton_b200.lora import grad_buffer, lora_grad_batch, lora_side
 
-    outs, saved = [], {}
+    outs, saved = [], {}      # saved: s . x . Aᵀ, and the factors as the GEMMs read them (A, B, Bᵀ)
     for group in GROUPS:
         x = acts[INPUT_OF[group[0]]]
         weights = [(layer[n]["packed"], layer[n]["state"]) for n in group]
         lora_on = [n for n in group if "A" in layer[n]]
         if lora_on:
-            downs = lora_down_batch([x] * len(lora_on), [layer[n]["A"] for n in lora_on], True,
-                                    [SCALING] * len(lora_on))
-            saved.update(zip(lora_on, downs))
-        xas = [saved.get(n) for n in group]
-        lbs = [layer[n]["B"] if n in saved else None for n in group]
+            side = lora_side([x] * len(lora_on), [layer[n]["A"] for n in lora_on], [SCALING] * len(lora_on),
+                             [layer[n]["B"] for n in lora_on], transpose=True)
+            saved.update(zip(lora_on, zip(*side)))
+        xas = [saved[n][0] if n in saved else None for n in group]
+        lbs = [saved[n][2] if n in saved else None for n in group]
         outs += linear_forward_group(x, weights, None, xas, lbs)
     for group in reversed(GROUPS):
         x = acts[INPUT_OF[group[0]]]
         weights = [(layer[n]["packed"], layer[n]["state"]) for n in group]
         dys = [acts["dy_" + n] for n in group]
         lora_on = [n for n in group if "A" in layer[n]]
-        ups = {}
+        ups, flat, zs = {}, None, []
+        for n in lora_on:
+            zs += [x, acts["dy_" + n]]
         if lora_on:
-            downs = lora_down_batch([acts["dy_" + n] for n in lora_on],
-                                    [layer[n]["B"] for n in lora_on], False, [SCALING] * len(lora_on))
+            flat = grad_buffer([(z,) for z in zs], x.device)
+            downs, *_ = lora_side([acts["dy_" + n] for n in lora_on], [saved[n][3] for n in lora_on],
+                                  [SCALING] * len(lora_on), zero=flat)
             ups.update(zip(lora_on, downs))
         us = [ups.get(n) for n in group]
-        las = [layer[n]["A"] if n in ups else None for n in group]
+        las = [saved[n][1] if n in ups else None for n in group]
         outs.append(linear_backward_dx_group(dys, weights, us, las))
         if lora_on:  # dA and dB of every adapter of the group in one launch
-            zs, ss, rms = [], [], []
+            ss, rms = [], []
             for n in lora_on:
-                zs += [x, acts["dy_" + n]]
-                ss += [ups[n], saved[n]]
+                ss += [ups[n], saved[n][0]]
                 rms += [True, False]
-            outs += lora_grad_batch(zs, ss, rms)
+            outs += lora_grad_batch(zs, ss, rms, flat)
     return outs
 
 
@@ -281,7 +283,7 @@ def layer_backward(layer, acts):
 def kernels_per_step(shapes, m):
     """Kernels of this library that one step launches: a fused GEMM per group and direction, one
     split-K reduction per output wherever the library's plan slices the contraction (the library
-    is asked), and lora_down / lora_grad twice each per LoRA projection."""
+    is asked), and per group with adapters the side work of either direction and the gradients."""
     import ctypes
 
     from hackaton_b200 import _lib
@@ -296,7 +298,7 @@ def kernels_per_step(shapes, m):
             if launches < 1:
                 raise RuntimeError(f"nf4b200_launches_group: {launches}")
             n += launches
-    # lora_down: one batched launch per group and direction; lora_grad: one per group
+    # lora_side: one launch per group and direction; lora_grad: one per group
     groups_with_lora = sum(1 for group in GROUPS if any(g in LORA_ON for g in group))
     return n + 3 * groups_with_lora
 
@@ -599,7 +601,7 @@ def run_leg(args):
     (193 MB of packed weights, more than the L2 holds) and nothing else: the small, bounded
     command the profiler captures are taken from. Prints one short JSON line."""
     from hackaton_b200 import _lib
-    from hackaton_b200.lora import lora_down_batch, lora_grad_batch
+    from hackaton_b200.lora import grad_buffer, lora_grad_batch, lora_side
     from hackaton_b200.nf4 import dequantize_nf4, linear_forward, prepare_weights
 
     device = torch.device("cuda", 0)
@@ -644,11 +646,12 @@ def run_leg(args):
         acts = make_activations(shapes, args.tokens or 2048, device)
         for i in range(reps * n_layers):
             lay = layers[i % n_layers]
-            xa = lora_down_batch([acts["x_attn"]] * 2, [lay["q"]["A"], lay["v"]["A"]], True, [SCALING] * 2)
-            u = lora_down_batch([acts["dy_q"], acts["dy_v"]], [lay["q"]["B"], lay["v"]["B"]], False,
-                                [SCALING] * 2)
-            lora_grad_batch([acts["x_attn"], acts["dy_q"], acts["x_attn"], acts["dy_v"]],
-                            [u[0], xa[0], u[1], xa[1]], [True, False, True, False])
+            zs = [acts["x_attn"], acts["dy_q"], acts["x_attn"], acts["dy_v"]]
+            flat = grad_buffer([(z,) for z in zs], device)
+            xa, _, _, bt = lora_side([acts["x_attn"]] * 2, [lay["q"]["A"], lay["v"]["A"]], [SCALING] * 2,
+                                     [lay["q"]["B"], lay["v"]["B"]], transpose=True)
+            u, *_ = lora_side([acts["dy_q"], acts["dy_v"]], bt, [SCALING] * 2, zero=flat)
+            lora_grad_batch(zs, [u[0], xa[0], u[1], xa[1]], [True, False, True, False], flat)
             launches += 3
     torch.cuda.synchronize()
     _lib.device_status()
@@ -836,7 +839,6 @@ def run_single(args):
 
     # ---- the step after q/k/v: rotation + grouped-query expansion, against the HBM roofline
     # (16,384 packed tokens of 4 sequences, 12 heads over 2 kv heads of 128: 218 MB per launch)
-    from hackaton_b200.rope import RotateGeometry, launch as rope_launch
     rp_n, rp_seq, rp_h, rp_kv, rp_d = 16384, 4096, 12, 2, 128
     rp_in = [[torch.randn(rp_n, hd * rp_d, device=device).half() for hd in (rp_h, rp_kv, rp_kv)] for _ in range(2)]
     rp_out = [[torch.empty(rp_n, rp_h, rp_d, device=device, dtype=torch.float16) for _ in range(3)] for _ in range(2)]
@@ -848,11 +850,12 @@ def run_single(args):
     rp_b = (torch.arange(rp_n, device=device) // rp_seq).to(torch.int32)
     rp_t = (torch.arange(rp_n, device=device) % rp_seq).to(torch.int32)
 
-    rp_geo = RotateGeometry(rp_n, rp_seq, rp_h, rp_kv, rp_d, False, 0, torch.float16)
-
     def rope_call(i, backward):
         src, dst = (rp_out[i % 2], rp_grad) if backward else (rp_in[i % 2], rp_out[i % 2])
-        rope_launch(src, dst, rp_cos, rp_sin, rp_b, rp_t, rp_geo, backward)
+        _lib.check(_lib.lib().nf4b200_qkv_rotate(
+            *(t.data_ptr() for t in (*src, *dst)), rp_cos.data_ptr(), rp_sin.data_ptr(), 0, rp_cos.stride(1),
+            rp_b.data_ptr(), rp_t.data_ptr(), rp_n, rp_seq, rp_h, rp_kv, rp_d, 0, int(backward), _lib.F16,
+            torch.cuda.current_stream().cuda_stream))
 
     rope_call(0, False)
     rope_call(1, False)
@@ -887,11 +890,12 @@ def run_single(args):
         ce[key] = {"us": us, "gbs": gbs, "frac_of_hbm": gbs / pk["hbm_gbs"], "bytes_per_element": bytes_per_elem}
     del ce_logits, ce_grad_out
 
-    # ---- the lm_head products of one chunk of the chunked loss (256 rows against the 151,936 x
-    # 1536 fp16 table: 467 MB, re-read from HBM by every launch) through the library's kernel,
-    # with torch's library GEMM timed beside them
+    # ---- the lm_head products of the chunked loss, in the rows that its gradient takes at a time (the 151,936
+    # x 1536 fp16 table, 467 MB, is re-read from HBM by every launch) through the library's kernel, with
+    # torch's library GEMM timed beside them
     from hackaton_b200.dense import fp16_linear
-    lm_rows, lm_hidden = 256, 1536
+    from hackaton_b200.lm_loss import CHUNK_TILE
+    lm_rows, lm_hidden = CHUNK_TILE, 1536
     lm_w = torch.randn(ce_vocab, lm_hidden, device=device, dtype=torch.float16)
     lm_w *= 0.02
     lm_h = [torch.randn(lm_rows, lm_hidden, device=device, dtype=torch.float16) for _ in range(2)]

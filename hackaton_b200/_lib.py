@@ -47,15 +47,6 @@ class Weight(Structure):
     ]
 
 
-class LoraItem(Structure):
-    """nf4b200_lora_item in include/nf4b200.h."""
-    _fields_ = [
-        ("in_", c_void_p), ("c", c_int64), ("ld_in", c_int64), ("p", c_void_p), ("out", c_void_p),
-        ("p16", c_void_p), ("b", c_void_p), ("b16", c_void_p), ("b16t", c_void_p), ("n", c_int64),
-        ("scaling", c_float), ("p_f32", c_int32), ("b_f32", c_int32), ("reserved", c_int32),
-    ]
-
-
 class Props(Structure):
     _fields_ = [("cc_major", c_int32), ("cc_minor", c_int32), ("sm_count", c_int32),
                 ("supported", c_int32), ("smem_per_block_optin", c_int64)]
@@ -108,7 +99,6 @@ def lib() -> ctypes.CDLL:
     pf = POINTER(c_float)
     handle.nf4b200_lora_down_batch.argtypes = [c_int, pv, c_int64, pi64, pi64, pv, pi64, pi64, pf,
                                                pv, c_void_p]
-    handle.nf4b200_lora_side.argtypes = [c_int, POINTER(LoraItem), c_int64, c_void_p, c_size_t, c_void_p]
     handle.nf4b200_lora_grad_batch.argtypes = [c_int, pv, pi64, pi64, pi64, pv, pv, pi64, pi64,
                                                c_void_p]
     handle.nf4b200_set_sm_limit.argtypes = [c_int]

@@ -8,40 +8,10 @@ forward, one backward, outputs fp16 with every k / v head repeated heads / kv_he
 
 from __future__ import annotations
 
-from dataclasses import dataclass
-
 import torch
 
 from . import _lib
 from ._autograd import call
-from .nf4 import _stream_ptr
-
-
-@dataclass
-class RotateGeometry:
-    """Everything about one rotation that is not a tensor."""
-    tokens: int
-    seq: int
-    heads: int
-    kv_heads: int
-    dim: int
-    padded: bool
-    batch_stride: int          # elements between the cos / sin tables of two batches, 0 if shared
-    proj_dtype: torch.dtype    # type of the projections (forward input, backward output)
-
-
-def launch(src, dst, cos, sin, b_idx, t_idx, geo: RotateGeometry, backward: bool):
-    """src, dst: (q, k, v) triples. Forward reads the projections and writes the expanded fp16
-    heads; backward reads the heads' gradients and writes the projections' gradients."""
-    device = dst[0].device
-    with torch.cuda.device(device):
-        _lib.check(_lib.lib().nf4b200_qkv_rotate(
-            src[0].data_ptr(), src[1].data_ptr(), src[2].data_ptr(),
-            dst[0].data_ptr(), dst[1].data_ptr(), dst[2].data_ptr(),
-            cos.data_ptr(), sin.data_ptr(), geo.batch_stride, cos.stride(1),
-            b_idx.data_ptr(), t_idx.data_ptr(), geo.tokens, geo.seq, geo.heads, geo.kv_heads,
-            geo.dim, int(geo.padded), int(backward),
-            _lib.F32 if geo.proj_dtype == torch.float32 else _lib.F16, _stream_ptr(device)))
 
 
 class _RotateOp:
