@@ -156,7 +156,7 @@ __device__ __forceinline__ void prefetch_span(const uint8_t* ptr, long long byte
 
 // Forward. A warp tile is MT * 16 weight rows of one member of the group (SWIGLU: the same 16 rows
 // of gate and of up) times up to 32 tokens; 2^split_log warps share a tile, each with a contiguous
-// slice of its k-blocks, and a CTA of 16 warps holds the other tiles of a set. Every warp brings its
+// slice of its k-blocks, and a CTA (of 16, 8 or 4 warps) holds the other tiles of a set. Every warp brings its
 // own codes and scales through a private ring in shared memory (cp.async), laid out [k-block][row]
 // [32 bytes], from which its fragments (rows g, g + 8; 8 bytes each) are read without conflicts: a
 // direct load of such a fragment touches eight lines, which cost as much of the L1 pipe as the

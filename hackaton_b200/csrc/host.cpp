@@ -58,7 +58,7 @@ py::bytes stamps(const Tensor& packed, const Tensor& absmax, const Tensor& code,
 Tensor rows_view(const Tensor& t, int64_t cols) {
     const auto aligned = [](const Tensor& v) { return (reinterpret_cast<uintptr_t>(v.const_data_ptr()) & 15) == 0; };
     Tensor v = t.dim() == 2 && t.size(1) == cols ? t : t.reshape({-1, cols});
-    if (v.stride(1) == 1 && v.stride(0) % 8 == 0 && aligned(v) && (v.size(0) <= 1 || v.stride(0) >= cols)) return v;
+    if (v.stride(1) == 1 && v.stride(0) % 8 == 0 && aligned(v) && v.stride(0) >= cols) return v;
     v = v.contiguous();
     // (a tensor that counts as contiguous keeps its address, and a single row its stride)
     if (cols % 8 == 0 && (!aligned(v) || v.stride(0) != cols)) v = v.clone(at::MemoryFormat::Contiguous);

@@ -267,8 +267,7 @@ def _rows_view(t, cols):
     """[..., cols] -> 2-D view with contiguous rows, 16-byte aligned and 8 elements apart (copying only
     if the layout forces it; columns that are no eights stay where they are)."""
     t2 = t.reshape(-1, cols)
-    if t2.stride(1) != 1 or t2.stride(0) % 8 != 0 or t2.data_ptr() % 16 != 0 or \
-            (t2.shape[0] > 1 and t2.stride(0) < cols):
+    if t2.stride(1) != 1 or t2.stride(0) % 8 != 0 or t2.data_ptr() % 16 != 0 or t2.stride(0) < cols:
         t2 = t2.contiguous()
         # (a tensor that counts as contiguous keeps its address, and a single row its stride)
         if cols % 8 == 0 and (t2.data_ptr() % 16 != 0 or t2.stride(0) != cols):

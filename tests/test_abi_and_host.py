@@ -430,11 +430,11 @@ def test_rows_view_gives_aligned_rows():
     kept = [flat[:320].view(5, 64), flat[8:328].view(5, 64), flat.view(16, 256)[:, 8:72], flat[:64].view(1, 64)]
     copied = [flat[1:321].view(5, 64), flat[3:67].view(1, 64), flat[8:].as_strided((1, 64), (67, 1)),
               flat.as_strided((4, 64), (67, 1)), flat[:320].view(64, 5).t(), flat[:64].expand(3, 64),
-              flat[1:65], flat[1:641].view(2, 5, 64)]
+              flat[1:65], flat[1:641].view(2, 5, 64), flat[:64].expand(1, 64)]
     for t in kept + copied:
         v = _rows_view(t, 64)
         assert torch.equal(v, t.reshape(-1, 64)) and v.stride(1) == 1 and v.stride(0) % 8 == 0
-        assert v.data_ptr() % 16 == 0 and (v.shape[0] == 1 or v.stride(0) >= 64)
+        assert v.data_ptr() % 16 == 0 and v.stride(0) >= 64
     assert all(_rows_view(t, 64).data_ptr() == t.data_ptr() for t in kept)
     odd = flat[1:1 + 5 * 63].view(5, 63)
     assert _rows_view(odd, 63).data_ptr() == odd.data_ptr()

@@ -213,6 +213,7 @@ def test_input_forms_of_the_calls(cuda_lib):
         "no rows": big[:0, 0, :k], "one row": big[0, :1, 8:8 + k],
         "contiguous at an odd address": big.flatten()[1:1 + 5 * k].view(5, k),
         "one row at an odd address": big.flatten()[3:3 + k].view(1, k),
+        "one row of stride 0": big[0, 0, :k].expand(1, k),
         "one row of an odd stride": big.flatten()[8:].as_strided((1, k), (k + 3, 1)),
     }
     outs = {
